@@ -612,104 +612,38 @@ void array_sums(ptyb_handle* h, const float2* g, const float2* hh, size_t n, int
 
 unsigned blocks_for(size_t n) { return (unsigned)((n + 255) / 256); }
 
-// In-place FFT of n complex doubles, forward, unscaled: radix 2 for a power of 2, else the
-// direct sum (sides 96 and 192, host-only work of the phase-ramp removal).
-void host_fft(std::vector<double>& re, std::vector<double>& im, size_t off, size_t stride, int n) {
-  if (n & (n - 1)) {
-    std::vector<double> r(n), i(n);
-    for (int k = 0; k < n; ++k) {
-      double sr = 0.0, si = 0.0;
-      for (int j = 0; j < n; ++j) {
-        const double a = -2.0 * M_PI * (double)((long long)j * k % n) / n;
-        const double c = std::cos(a), s = std::sin(a);
-        const double xr = re[off + j * stride], xi = im[off + j * stride];
-        sr += xr * c - xi * s;
-        si += xr * s + xi * c;
-      }
-      r[k] = sr;
-      i[k] = si;
-    }
-    for (int k = 0; k < n; ++k) {
-      re[off + k * stride] = r[k];
-      im[off + k * stride] = i[k];
-    }
-    return;
-  }
-  std::vector<double> r(n), i(n);
-  for (int k = 0; k < n; ++k) {
-    r[k] = re[off + k * stride];
-    i[k] = im[off + k * stride];
-  }
-  for (int a = 1, j = 0; a < n; ++a) {
-    int bit = n >> 1;
-    for (; j & bit; bit >>= 1) j ^= bit;
-    j ^= bit;
-    if (a < j) {
-      std::swap(r[a], r[j]);
-      std::swap(i[a], i[j]);
-    }
-  }
-  for (int len = 2; len <= n; len <<= 1) {
-    const double ang = -2.0 * M_PI / len;
-    for (int s0 = 0; s0 < n; s0 += len)
-      for (int k = 0; k < len / 2; ++k) {
-        const double wr = std::cos(ang * k), wi = std::sin(ang * k);
-        const int u = s0 + k, v = s0 + k + len / 2;
-        const double tr = r[v] * wr - i[v] * wi, ti = r[v] * wi + i[v] * wr;
-        r[v] = r[u] - tr;
-        i[v] = i[u] - ti;
-        r[u] += tr;
-        i[u] += ti;
-      }
-  }
-  for (int k = 0; k < n; ++k) {
-    re[off + k * stride] = r[k];
-    im[off + k * stride] = i[k];
-  }
-}
-
 // PyNX ZeroPhaseRamp (engine/ptycho.rs:1134-1170): the centroid of the probe modes' summed
-// far-field intensity on the host, then the probe's and the object's phase ramps on the device.
+// far-field intensity, in double, then the probe's and the object's phase ramps. All of it on
+// the device and the handle's stream (ramp_rows_kernel), about 60 us: with the probe brought to
+// the host and transformed there a call took 10.5 ms longer at 256² x 2 modes and 237 ms at
+// 192², where no radix-2 transform runs.
 void zero_phase_ramp(ptyb_handle* h) {
   const int N = h->N;
   const size_t plane = (size_t)N * N;
-  std::vector<float2> pr((size_t)h->K * plane);
-  check(h, cudaMemcpyAsync(pr.data(), h->probe, pr.size() * sizeof(float2), cudaMemcpyDeviceToHost,
-                           h->stream),
-        "probe");
-  check(h, cudaStreamSynchronize(h->stream), "probe");
-  std::vector<double> v(plane, 0.0), re(plane), im(plane);
-  for (int m = 0; m < h->K; ++m) {
-    // far = FFT of the probe in the shifted layout
-    for (int jy = 0; jy < N; ++jy)
-      for (int jx = 0; jx < N; ++jx) {
-        const float2 p = pr[m * plane + (size_t)((jy + N / 2) % N) * N + (jx + N / 2) % N];
-        re[(size_t)jy * N + jx] = p.x;
-        im[(size_t)jy * N + jx] = p.y;
-      }
-    for (int y = 0; y < N; ++y) host_fft(re, im, (size_t)y * N, 1, N);
-    for (int x = 0; x < N; ++x) host_fft(re, im, x, N, N);
-    // v at natural i = |far[shift(i)]|²
-    for (int iy = 0; iy < N; ++iy)
-      for (int ix = 0; ix < N; ++ix) {
-        const size_t j = (size_t)((iy + N / 2) % N) * N + (ix + N / 2) % N;
-        v[(size_t)iy * N + ix] += re[j] * re[j] + im[j] * im[j];
-      }
+  if (!h->ramp_rows) {
+    h->ramp_rows = alloc<double2>(h, (size_t)h->K * plane);
+    h->ramp_sums = alloc<double>(h, (size_t)h->K * N * 3 + 2);
   }
-  double w = 0.0, wy = 0.0, wx = 0.0;
-  for (size_t i = 0; i < plane; ++i) {
-    w += v[i];
-    wy += v[i] * (double)(i / N);
-    wx += v[i] * (double)(i % N);
-  }
-  const double dy = wy / w - (double)(N / 2), dx = wx / w - (double)(N / 2);
+  double* shift = h->ramp_sums + (size_t)h->K * N * 3;
+  const dim3 lines(N, h->K);
+  const size_t smem = 2 * (size_t)N * sizeof(double2);
+  timed(h, kKMisc, [&] { ramp_rows_kernel<<<lines, N, smem, h->stream>>>(h->probe, N, h->ramp_rows); });
+  launched(h, "probe far field rows");
+  timed(h, kKMisc, [&] {
+    ramp_columns_kernel<<<lines, N, smem, h->stream>>>(h->ramp_rows, N, h->ramp_sums);
+  });
+  launched(h, "probe far field columns");
+  timed(h, kKMisc, [&] {
+    ramp_centroid_kernel<<<1, 32, 0, h->stream>>>(h->ramp_sums, h->K * N, N, shift);
+  });
+  launched(h, "probe far field centroid");
   const size_t np = (size_t)h->K * plane, no = (size_t)h->nobj * h->nyo * h->nxo;
   timed(h, kKMisc, [&] {
-    ramp_kernel<<<blocks_for(np), 256, 0, h->stream>>>(h->probe, h->K, N, N, dy, dx, N, N, -1.0);
+    ramp_kernel<<<blocks_for(np), 256, 0, h->stream>>>(h->probe, h->K, N, N, shift, N, N, -1.0);
   });
   launched(h, "probe ramp");
   timed(h, kKMisc, [&] {
-    ramp_kernel<<<blocks_for(no), 256, 0, h->stream>>>(h->object, h->nobj, h->nyo, h->nxo, dy, dx,
+    ramp_kernel<<<blocks_for(no), 256, 0, h->stream>>>(h->object, h->nobj, h->nyo, h->nxo, shift,
                                                       N, N, 1.0);
   });
   launched(h, "object ramp");

@@ -161,6 +161,10 @@ struct ptyb_handle {
   double* pcg_norms = nullptr;    // [P][K]
   double* pcg_modes = nullptr;    // [K][2]
   double* partials = nullptr;    // [kPartialBlocks][2]
+  // Phase-ramp removal: the probe's row transforms [K][N][N], the columns' sums [K·N][3] and
+  // the centroid's offset (dy, dx) behind them.
+  double2* ramp_rows = nullptr;
+  double* ramp_sums = nullptr;
   std::vector<ptyb::eng::Buf> bufs;
   // Per-kernel device timing (CUDA events on the engine's stream), when enabled.
   bool timing = false;

@@ -192,10 +192,97 @@ static __global__ void scale_kernel(float2* x, float s, size_t n) {
   x[i] = cscale(x[i], s);
 }
 
+// The centroid of the probe's far field for `zero_phase_ramp` (engine/ptycho.rs:1134-1152), in
+// double: one block per line, thread k taking X[k] = Σ_j x[j]·e^{−2πi·jk/N} as the direct sum
+// over a table of N twiddles in shared memory. K·N² outputs of N terms (33.5 M complex FMAs per
+// direction at 256² x 2) take about 20 µs a direction, so no fast transform in double is worth
+// its code here. The plane is not shifted before the transform: a shift changes
+// the spectrum's phases and not its modulus.
+PTYB_D double2 dft_line_term(const double2* x, const double2* w, int N) {
+  double2 s = make_double2(0.0, 0.0);
+  int i = 0;
+  const int k = threadIdx.x;
+#pragma unroll 4
+  for (int j = 0; j < N; ++j) {
+    const double2 a = x[j], b = w[i];
+    s.x += a.x * b.x - a.y * b.y;
+    s.y += a.x * b.y + a.y * b.x;
+    i += k;
+    if (i >= N) i -= N;
+  }
+  return s;
+}
+
+PTYB_D void dft_line_twiddles(double2* w, int N) {
+  double sn, cs;
+  sincospi(-2.0 * threadIdx.x / N, &sn, &cs);
+  w[threadIdx.x] = make_double2(cs, sn);
+}
+
+// Block (y, m), N threads: rows[m][y][k].
+static __global__ void __launch_bounds__(256) ramp_rows_kernel(const float2* probe, int N,
+                                                               double2* rows) {
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  double2* x = reinterpret_cast<double2*>(smem_raw);
+  const size_t line = ((size_t)blockIdx.y * N + blockIdx.x) * N;
+  const float2 v = probe[line + threadIdx.x];
+  x[threadIdx.x] = make_double2(v.x, v.y);
+  dft_line_twiddles(x + N, N);
+  __syncthreads();
+  rows[line + threadIdx.x] = dft_line_term(x, x + N, N);
+}
+
+// Block (kx, m), N threads: with v(ky) = |F(ky, kx)|², Σ v, Σ v·iy and Σ v·ix over the column at
+// the natural indices iy = (ky + N/2) % N, ix, into sums[m·N + kx][3].
+static __global__ void __launch_bounds__(256) ramp_columns_kernel(const double2* rows, int N,
+                                                                  double* sums) {
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  __shared__ double red[2][8];
+  double2* x = reinterpret_cast<double2*>(smem_raw);
+  const int kx = blockIdx.x, t = threadIdx.x;
+  x[t] = rows[((size_t)blockIdx.y * N + t) * N + kx];
+  dft_line_twiddles(x + N, N);
+  __syncthreads();
+  const double2 f = dft_line_term(x, x + N, N);
+  const double v = f.x * f.x + f.y * f.y;
+  const double s0 = warp_sum(v), s1 = warp_sum(v * (double)((t + N / 2) % N));
+  if (t % 32 == 0) {
+    red[0][t / 32] = s0;
+    red[1][t / 32] = s1;
+  }
+  __syncthreads();
+  if (t == 0) {
+    double a = 0.0, b = 0.0;
+    for (int w = 0; w < N / 32; ++w) {
+      a += red[0][w];
+      b += red[1][w];
+    }
+    double* out = sums + ((size_t)blockIdx.y * N + kx) * 3;
+    out[0] = a;
+    out[1] = b;
+    out[2] = a * (double)((kx + N / 2) % N);
+  }
+}
+
+// shift = centroid − N/2 along y and x from the columns' sums, one warp, fixed order.
+static __global__ void __launch_bounds__(32) ramp_centroid_kernel(const double* sums, int n,
+                                                                  int N, double* shift) {
+  double s[3] = {0.0, 0.0, 0.0};
+  for (int i = threadIdx.x; i < n; i += 32)
+    for (int k = 0; k < 3; ++k) s[k] += sums[(size_t)i * 3 + k];
+  for (int k = 0; k < 3; ++k) s[k] = warp_sum(s[k]);
+  if (threadIdx.x == 0) {
+    shift[0] = s[1] / s[0] - (double)(N / 2);
+    shift[1] = s[2] / s[0] - (double)(N / 2);
+  }
+}
+
 // x[k][y][x] *= exp(i·2π·sign·(dy·(y − hy)/sy + dx·(x − hx)/sx)) for every plane k
-// (the ramps of `zero_phase_ramp`, engine/ptycho.rs:1153-1170), phase in double.
-static __global__ void ramp_kernel(float2* x, int nplanes, int ny, int nx, double dy, double dx,
-                            double sy, double sx, double sign) {
+// (the ramps of `zero_phase_ramp`, engine/ptycho.rs:1153-1170) with (dy, dx) = shift, phase in
+// double.
+static __global__ void ramp_kernel(float2* x, int nplanes, int ny, int nx, const double* shift,
+                                   double sy, double sx, double sign) {
+  const double dy = shift[0], dx = shift[1];
   const size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
   const size_t n = (size_t)nplanes * ny * nx;
   if (i >= n) return;
