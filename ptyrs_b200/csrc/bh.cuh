@@ -31,7 +31,7 @@ struct BhArgs {
   double* out;            // [slot]: the frame's share of H(u, v)
   int nyo, nxo, nprobe, nobj;
   int same;               // v is u: one tangent transform per mode
-  // U psi of every slot and mode as the gradient pass kept it, [slot][K][kx][ky] (the frame
+  // U psi of every slot and mode as the gradient pass kept it, [slot][K][ky][kx] (the frame
   // kernel's unnormalised transform), and its exit-plane field g = Uᴴ(2·td), [slot][K][N][N].
   const float2* psi;
   const float2* g;
@@ -84,7 +84,7 @@ __global__ void __launch_bounds__(FrameShape<N, C>::T, 1) bh_hessian_kernel(BhAr
   double gterm = 0.0;
   for (int m = 0; m < K; ++m) {
     const int pm = m % a.nprobe, om = m / a.nprobe;
-    const float2* po_m = a.psi + ((size_t)slot * K + m) * N * N + (size_t)r * H * N;
+    const float2* po_m = a.psi + ((size_t)slot * K + m) * N * N + r * H;
     const float2* g_m = a.g + ((size_t)slot * K + m) * N * N;
     // Exit-plane rows (shifted, as the frame kernel's) of J u and J v; J″(u, v) against g.
 #pragma unroll 2
@@ -132,8 +132,8 @@ __global__ void __launch_bounds__(FrameShape<N, C>::T, 1) bh_hessian_kernel(BhAr
     // Columns kx = r·H + c, elements ky: Σ|U psi|², Re(conj(L_u)·L_v), c_u and c_v terms.
 #pragma unroll 2
     for (int idx = tid; idx < H * N; idx += T) {
-      const int c = idx / N, ky = idx % N;
-      const float2 po = po_m[(size_t)c * N + ky];
+      const int c = idx % H, ky = idx / H;
+      const float2 po = po_m[(size_t)ky * N + c];
       const float2 lu = S1[c * L + (ky ^ swz(c))];
       const float2 lv = a.same ? lu : S1[(H + c) * L + (ky ^ swz(H + c))];
       acc[c * AS + ky] += cnorm2(po) * inv_n2;

@@ -15,7 +15,20 @@ PTYB_HD float2 cmul(float2 a, float2 b) {
 PTYB_HD float2 cmulc(float2 a, float2 b) {
   return make_float2(a.x * b.x + a.y * b.y, a.x * b.y - a.y * b.x);
 }
+// a * b and conj(a) * b in the line transforms and around them: the products that are rounded
+// and those that are fused are written out, so the result does not depend on what the compiler
+// makes of the code around.
+PTYB_D float2 cmul_rn(float2 a, float2 b) {
+  return make_float2(fmaf(a.x, b.x, -(a.y * b.y)), fmaf(a.x, b.y, a.y * b.x));
+}
+PTYB_D float2 cmulc_rn(float2 a, float2 b) {
+  return make_float2(fmaf(a.x, b.x, a.y * b.y), fmaf(a.x, b.y, -(a.y * b.x)));
+}
 PTYB_HD float2 cscale(float2 a, float s) { return make_float2(a.x * s, a.y * s); }
+// The same, not contracted into an addition that follows.
+PTYB_D float2 cscale_rn(float2 a, float s) {
+  return make_float2(__fmul_rn(a.x, s), __fmul_rn(a.y, s));
+}
 PTYB_HD float2 cconj(float2 a) { return make_float2(a.x, -a.y); }
 PTYB_HD float cnorm2(float2 a) { return a.x * a.x + a.y * a.y; }
 

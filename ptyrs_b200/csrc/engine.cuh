@@ -118,7 +118,7 @@ struct ptyb_handle {
   float2* spec = nullptr;        // [K][N][N]
   float2* spec_d = nullptr;      // [K][N][N]
   float2* wave_all = nullptr;    // [P][K][N][N]
-  // ML: every frame's detector field of one cycle's gradient pass, [P][K][kx][ky], and the
+  // ML: every frame's detector field of one cycle's gradient pass, [P][K][ky][kx], and the
   // probe gradient's summed spectrum under the position model.
   float2* psi_all = nullptr;
   float2* g_all = nullptr;         // [P][K][N][N] the gradient pass's exit-plane field g

@@ -25,6 +25,14 @@ PTYB_HD constexpr float cos16(int t) {
   }
 }
 
+// x·(c + i·s) with c and s known at compile time. Which product of a component is rounded and
+// which fused is fixed here, by the signs: on transforms of hard-edged apertures, whose far-field
+// zeros cancel to the last bit, this choice measured closer to 64 bits than the others.
+PTYB_D float2 rotate_by(float2 x, float c, float s) {
+  return make_float2(c < 0.f && s < 0.f ? fmaf(-x.y, s, x.x * c) : fmaf(x.x, c, -(x.y * s)),
+                     c < 0.f ? fmaf(x.y, c, x.x * s) : fmaf(x.x, s, x.y * c));
+}
+
 // x · e^{DIR·2πi·t/R} with DIR = -1 (forward) or +1 (inverse); t and R compile-time after
 // unrolling, so the trivial rotations cost no multiply.
 template <int R, int DIR>
@@ -36,7 +44,7 @@ PTYB_D float2 rotate(float2 x, int t) {
   if (t16 == 12) return DIR < 0 ? make_float2(-x.y, x.x) : make_float2(x.y, -x.x);
   const float c = cos16(t16);
   const float s = DIR * cos16(t16 + 12);  // DIR·sin(2πt/16)
-  return make_float2(x.x * c - x.y * s, x.x * s + x.y * c);
+  return rotate_by(x, c, s);
 }
 
 template <int R>
@@ -57,8 +65,8 @@ PTYB_D void dft_stages(float2 (&x)[R]) {
     for (int k = 0; k < R; k += 2 * HALF) {
 #pragma unroll
       for (int j = 0; j < HALF; ++j) {
-        const float2 b = rotate<2 * HALF, DIR>(x[k + j + HALF], j);
         const float2 a = x[k + j];
+        const float2 b = rotate<2 * HALF, DIR>(x[k + j + HALF], j);
         x[k + j] = cadd(a, b);
         x[k + j + HALF] = csub(a, b);
       }
@@ -92,7 +100,7 @@ PTYB_D float2 rotate24(float2 x, int t) {
   if (t % 24 == 0) return x;
   const float c = cos24(t);
   const float s = DIR * cos24(t - 6);  // DIR·sin(2πt/24)
-  return make_float2(x.x * c - x.y * s, x.x * s + x.y * c);
+  return rotate_by(x, c, s);
 }
 
 template <int R, int DIR>
@@ -194,7 +202,7 @@ PTYB_D void line_fft(float2* line, int t, const LineTwiddles<N>& tw, int sw) {
   for (int n1 = 0; n1 < N1; ++n1) v[n1] = line[(N2 * n1 + t) ^ sw];
   dft<N1, DIR>(v);
 #pragma unroll
-  for (int k1 = 1; k1 < N1; ++k1) v[k1] = cmul(v[k1], DIR < 0 ? tw.w[k1] : cconj(tw.w[k1]));
+  for (int k1 = 1; k1 < N1; ++k1) v[k1] = cmul_rn(DIR < 0 ? tw.w[k1] : cconj(tw.w[k1]), v[k1]);
   __syncwarp();
 #pragma unroll
   for (int k1 = 0; k1 < N1; ++k1) line[(k1 * N2 + ((t + k1) & (N2 - 1))) ^ sw] = v[k1];

@@ -2,14 +2,21 @@
 // inverse 2-D FFT → exit-wave update, for every probe mode of one diffraction frame, on one
 // thread-block cluster whose distributed shared memory holds the frame's K planes.
 //
-// Cluster of C CTAs, CTA rank r owning H = N/C rows. Shared memory holds K·H lines of N
-// float2, each XOR-swizzled (`swz`) so no access pattern conflicts on banks. The row FFTs run
-// on rows; a
-// cluster-wide transpose through DSMEM turns the rows into H columns per CTA, stored as lines,
-// so the column FFTs, the per-pixel projection (which needs every mode at a pixel) and the
-// inverse column FFTs run on local lines; a second transpose brings the rows back for the
-// inverse row FFTs and the epilogue. Nothing but the object window, the counts and the output
-// touches global memory.
+// Cluster of C CTAs, CTA rank r owning H = N/C rows, then columns (plane.cuh): each thread loads
+// its elements of a row into registers and forms the exit wave there, the row FFTs leave their
+// spectra in shared memory, the transpose reads them from the other CTAs' shared memory straight
+// into the column FFTs' registers, and the per-pixel projection (which needs every mode at a
+// pixel: the modes but the last wait in shared memory) runs on the column in registers between
+// the forward and the inverse FFT; the way back is the same. Nothing but the object window, the
+// probes, the counts and the output touches global memory.
+//
+// What bounds it: latency. The exit waves' loads, the exchanges and the cluster barriers around
+// the transposes leave 37 % of the issue slots busy at 16 warps per SM (256² x 2), the memory
+// system under 25 %. Against the form it replaces (planes in shared memory for every step: 13
+// reads and 12 writes of each element per pass instead of 6.5 and 6.5, four global loads in
+// flight instead of 16) the passes take, per frame on one B200: gradient 256² x 2 3.53 -> 2.0 us,
+// carry 4.17 -> 2.27, LSQML 128² x 3 forward 0.77 -> 0.49 and backward 1.06 -> 0.63, amplitude
+// 96² x 2 0.83 -> 0.49, gradient 192² 1.53 -> 0.64, rPIE 64² 36 -> 13.5 us per batch of 100.
 //
 // Reference operators followed (physwkim/ptyrs): exit wave `obj_probe_to_psi`
 // (engine/ops.rs:47-71), unitary FFT (engine/fft.rs:155-234), the rPIE modulus
@@ -21,6 +28,7 @@
 
 #include "common.cuh"
 #include "fft.cuh"
+#include "plane.cuh"
 
 namespace cg = cooperative_groups;
 
@@ -70,8 +78,7 @@ struct FrameArgs {
   // per-frame (moved) probes of the position model.
   int probe_stride;
   // kMlGrad, optional: the detector field Ψ = DFT(P·O·q) of every mode kept for the line
-  // search and the magnitude projection, [slot][K][kx][ky] (columns contiguous); kProjectKept
-  // reads it back.
+  // search and the magnitude projection, [slot][K][ky][kx]; kProjectKept reads it back.
   float2* psi_out;
   // kCarry (AP, DM, RAAR; engine/ptycho.rs:609-730): the carried exit waves `carry` and RAAR's
   // iterate `iter` of the launch's frames, [slot][K][N][N] natural layout. The projection's
@@ -189,12 +196,12 @@ PTYB_D double batch_mean(const float* v, const int* frames, int by_frame, int ns
   return *slot;
 }
 
-// Cluster-wide sums of two doubles (every CTA gets the totals, added in rank order).
-template <int N, int C>
+// Cluster-wide sums of two doubles over CTAs of T threads (every CTA gets the totals, added in
+// rank order).
+template <int T, int C>
 PTYB_D void cluster_sum2(double& x, double& y, double* red, cg::cluster_group& cluster) {
-  using F = FrameShape<N, C>;
   double v[4] = {x, y, 0.0, 0.0};
-  block_sum<F::T>(v, 2, red);
+  block_sum<T>(v, 2, red);
   csync<C>(cluster);
   double sx = 0.0, sy = 0.0;
   for (int q = 0; q < C; ++q) {
@@ -208,10 +215,9 @@ PTYB_D void cluster_sum2(double& x, double& y, double* red, cg::cluster_group& c
 }
 
 // Cluster-wide sums of four doubles, every thread getting them (rank order, as cluster_sum2).
-template <int N, int C>
+template <int T, int C>
 PTYB_D void cluster_sum4(double (&v)[4], double* red, cg::cluster_group& cluster) {
-  using F = FrameShape<N, C>;
-  block_sum<F::T>(v, 4, red);
+  block_sum<T>(v, 4, red);
   csync<C>(cluster);
   double t[4] = {0.0, 0.0, 0.0, 0.0};
   for (int q = 0; q < C; ++q) {
@@ -224,141 +230,162 @@ PTYB_D void cluster_sum4(double (&v)[4], double* red, cg::cluster_group& cluster
   for (int k = 0; k < 4; ++k) v[k] = t[k];
 }
 
-// The projection's input S = c_po·po + c_psi·carry + c_it·iter at element `pix` of mode m of
-// `slot` (kCarry); the prologue (`store`) also writes it to RAAR's iterate.
-template <int N>
-PTYB_D float2 carry_mix(const FrameArgs& a, float2 po, int slot, int m, int pix, int K,
-                        bool store) {
-  const size_t gi = ((size_t)slot * K + m) * N * N + pix;
-  float2 v = cscale(po, a.c_po);
-  if (a.c_psi != 0.f) v = cadd(v, cscale(a.carry[gi], a.c_psi));
-  if (a.c_it != 0.f) v = cadd(v, cscale(a.iter[gi], a.c_it));
-  if (store && a.iter) a.iter[gi] = v;
-  return v;
+// The projection's input S = c_po·po + c_psi·carry + c_it·iter (kCarry) in place of po at a
+// thread's row-mapped elements, `base` the offset of the first one in the carried planes; the
+// prologue (`store`) also writes it to RAAR's iterate.
+template <int N, int C>
+PTYB_D void carry_mix(const FrameArgs& a, float2 (&v)[PlaneShape<N, C>::E], size_t base,
+                      bool store) {
+  using F = PlaneShape<N, C>;
+  auto xof = [](int i) { return F::G * ((i + F::E / 2) % F::E); };
+#pragma unroll
+  for (int i = 0; i < F::E; ++i) v[i] = cscale(v[i], a.c_po);
+  if (a.c_psi != 0.f) {
+    const float2* src = a.carry + base;
+#pragma unroll
+    for (int i = 0; i < F::E; ++i) v[i] = cadd(v[i], cscale(src[xof(i)], a.c_psi));
+  }
+  if (a.c_it != 0.f) {
+    const float2* src = a.iter + base;
+#pragma unroll
+    for (int i = 0; i < F::E; ++i) v[i] = cadd(v[i], cscale(src[xof(i)], a.c_it));
+  }
+  if (store && a.iter) {
+    float2* dst = a.iter + base;
+#pragma unroll
+    for (int i = 0; i < F::E; ++i) dst[xof(i)] = v[i];
+  }
 }
 
 template <int N, int C, int MODE>
-__global__ void __launch_bounds__(FrameShape<N, C>::T,
-                                  N == 256 && FrameShape<N, C>::T <= 256 &&
-                                          (MODE == kMlGrad || MODE == kBhGrad ||
-                                           MODE == kProjectKept ||
-                                           MODE == kLlk || MODE == kCarry)
-                                      ? 3
-                                      : frame_min_blocks<N, C>())
+__global__ void __launch_bounds__(PlaneShape<N, C>::T, plane_min_blocks<N, C>())
     frame_kernel(FrameArgs a) {
-  using F = FrameShape<N, C>;
-  constexpr int H = F::H, T = F::T, L = F::L;
-  extern __shared__ __align__(16) unsigned char smem_raw[];
+  using L = Lines<N, C>;
+  constexpr int H = L::H, T = L::T, E = L::N1, N2 = L::N2;
+  extern __shared__ __align__(128) unsigned char plane_smem[];
   const int K = a.nprobe * a.nobj;
-  float2* S = reinterpret_cast<float2*>(smem_raw);
-  float2* tw = S + (size_t)K * H * L;
-  double* red = reinterpret_cast<double*>(tw + N);  // 8 results + [T/32 ≤ 32][4] partials
+  float2* S = reinterpret_cast<float2*>(plane_smem);
+  float2* table = S + (size_t)K * H * N;
+  double* red = reinterpret_cast<double*>(table + N);  // 8 results + [T/32 ≤ 32][4] partials
   cg::cluster_group cluster = cg::this_cluster();
   const int r = C > 1 ? (int)cluster.block_rank() : 0;
   const int slot = blockIdx.x / C;
   const int f = a.frames[slot];
   const int2 corner = a.corners[f];
   const int tid = threadIdx.x;
-  LineTwiddles<N> ltw;
-  ltw.load(a.tw, tid % F::G);
-  (void)tw;
+  const L ln(S, table, r);
+  L::fill_table(table, a.tw);
+  constexpr size_t plane = (size_t)N * N;
+  constexpr bool from_field = MODE == kFromStore || MODE == kProjectKept;
 
-  float omax = 0.f;
-  if (MODE == kFromStore) {
-    const float2* src = a.field + ((size_t)slot * C + r) * K * H * N;
-#pragma unroll 8
-    for (int idx = tid; idx < K * H * N; idx += T) {
-      const int line = idx / N, e = idx % N;
-      S[line * L + (e ^ swz(line))] = src[idx];
+  // Row-mapped: the row's natural index and its first element; element i of the thread is the
+  // shifted column N2·i + rt, natural column N2·((i + E/2) % E) + rt.
+  const int ny = (r * H + ln.y + N / 2) % N;
+  const int rpix = ny * N + ln.rt;
+  auto xof = [](int i) { return N2 * ((i + E / 2) % E); };
+  // O·q of the row under object mode om; `omax` takes the largest |O|².
+  auto window = [&](float2 (&oq)[E], int om, float& omax) {
+    const float2* o = a.object + ((size_t)om * a.nyo + corner.x + ny) * a.nxo + corner.y + ln.rt;
+    const float2* q = a.quad + rpix;
+#pragma unroll
+    for (int i = 0; i < E; ++i) oq[i] = o[xof(i)];
+#pragma unroll
+    for (int i = 0; i < E; ++i) {
+      if (MODE == kRpie) omax = fmaxf(omax, cnorm2(oq[i]));
+      oq[i] = cmul_rn(oq[i], q[xof(i)]);
     }
-  } else if (MODE == kProjectKept) {
-    // this CTA's columns of the kept Ψ, [slot][m][kx][ky]
-    const float2* src = a.psi_out + (size_t)slot * K * N * N;
-#pragma unroll 8
-    for (int idx = tid; idx < K * H * N; idx += T) {
-      const int line = idx / N, e = idx % N, m = line / H, c = line % H;
-      S[line * L + (e ^ swz(line))] = src[((size_t)m * N + r * H + c) * N + e];
-    }
-  } else {
-    // Exit waves ψ = P·O·q of shifted rows r·H .. r·H+H-1, every mode; the object window and
-    // the phase are read once per pixel.
-#pragma unroll 2
-    for (int idx = tid; idx < H * N; idx += T) {
-      const int yl = idx / N, jx = idx % N;
-      const int ny = (r * H + yl + N / 2) % N, nx = (jx + N / 2) % N;
-      const float2 q = a.quad[ny * N + nx];
-      for (int om = 0; om < a.nobj; ++om) {
-        const float2 o = a.object[((size_t)om * a.nyo + corner.x + ny) * a.nxo + corner.y + nx];
-        const float2 oq = cmul(o, q);
-        if (MODE == kRpie && om == 0) omax = fmaxf(omax, cnorm2(o));
-        for (int pm = 0; pm < a.nprobe; ++pm) {
-          const int line = (om * a.nprobe + pm) * H + yl;
-          // (P·O)·q as P·(O·q): the reference's product up to rounding
-          float2 v =
-              cmul(a.probe[(size_t)slot * a.probe_stride + ((size_t)pm * N + ny) * N + nx], oq);
-          if (MODE == kCarry)
-            v = carry_mix<N>(a, v, slot, om * a.nprobe + pm, ny * N + nx, K, true);
-          S[line * L + (jx ^ swz(line))] = v;
-        }
+  };
+
+  float2 v[E];
+  if (!from_field) {
+    // Exit waves ψ = P·O·q of the rows, mode by mode; (P·O)·q as P·(O·q): the reference's
+    // product up to rounding.
+    float2 oq[E];
+    float omax = 0.f;
+#pragma unroll 1
+    for (int m = 0, om = 0, pm = 0; m < K; ++m) {
+      if (pm == 0) window(oq, om, omax);
+      const float2* p = a.probe + (size_t)slot * a.probe_stride + pm * plane + rpix;
+#pragma unroll
+      for (int i = 0; i < E; ++i) v[i] = p[xof(i)];
+#pragma unroll
+      for (int i = 0; i < E; ++i) v[i] = cmul_rn(v[i], oq[i]);
+      if (MODE == kCarry)
+        carry_mix<N, C>(a, v, ((size_t)slot * K + m) * plane + rpix, true);
+      if (m == 0) __syncthreads();  // the twiddle table
+      ln.rows_forward(v, m);
+      if (++pm == a.nprobe) {
+        pm = 0;
+        ++om;
       }
     }
-  }
-  __syncthreads();
-
-  if (MODE == kRpie) {
-    // max |O|² over the window: block max, then across the cluster in rank order.
-    omax = warp_max(omax);
-    float* fred = reinterpret_cast<float*>(red + 8);
-    if (tid % 32 == 0) fred[tid / 32] = omax;
-    __syncthreads();
-    if (tid == 0) {
-      float mx = 0.f;
-      for (int q = 0; q < T / 32; ++q) mx = fmaxf(mx, fred[q]);
-      reinterpret_cast<float*>(red)[0] = mx;
+    if (MODE == kRpie) {
+      // max |O|² over the window: block max, then across the cluster in rank order.
+      omax = warp_max(omax);
+      float* fred = reinterpret_cast<float*>(red + 8);
+      if (tid % 32 == 0) fred[tid / 32] = omax;
+      __syncthreads();
+      if (tid == 0) {
+        float mx = 0.f;
+        for (int q = 0; q < T / 32; ++q) mx = fmaxf(mx, fred[q]);
+        reinterpret_cast<float*>(red)[0] = mx;
+      }
     }
-  }
-
-  if (MODE != kFromStore && MODE != kProjectKept) {
-    all_lines<N, C, -1>(S, K * H, ltw);
-    transpose<N, C>(S, K, cluster);  // its first cluster barrier publishes red[0]
+    L::publish();
     if (MODE == kRpie && r == 0 && tid == 0) {
       float mx = 0.f;
       for (int q = 0; q < C; ++q)
         mx = fmaxf(mx, *reinterpret_cast<float*>(C > 1 ? cluster.map_shared_rank(red, q) : red));
       a.omax[slot] = mx;
     }
-    all_lines<N, C, -1>(S, K * H, ltw);
   }
 
-  if ((MODE == kMlGrad || MODE == kBhGrad) && a.psi_out) {
-    // Ψ of this CTA's columns to [slot][m][kx][ky]
-    float2* dst = a.psi_out + (size_t)slot * K * N * N;
-#pragma unroll 8
-    for (int idx = tid; idx < K * H * N; idx += T) {
-      const int line = idx / N, e = idx % N, m = line / H, c = line % H;
-      dst[((size_t)m * N + r * H + c) * N + e] = S[line * L + (e ^ swz(line))];
+  // Detector plane, column-mapped: element i is the pixel (ky, kx) = (N2·i + t, r·H + c).
+  // Unnormalised transforms: Ψ_ortho = Ψ/N, and the inverse of the update takes a 1/N more.
+  constexpr float inv_n2 = 1.0f / ((float)N * (float)N);
+  const int kx = r * H + ln.c, dpix = ln.t * N + kx;
+  constexpr int kRow = N2 * N;  // pixels between a thread's elements
+  float yo[E], ic[E];
+  {
+    const float* iobs = a.iobs + (size_t)f * plane + dpix;
+#pragma unroll
+    for (int i = 0; i < E; ++i) {
+      yo[i] = iobs[i * kRow];
+      ic[i] = 0.f;
     }
   }
-
-  // Detector plane: CTA r holds columns r·H .. r·H+H-1 as lines (m·H + c), elements ky.
-  // Unnormalised transforms: Ψ_ortho = S/N, and the inverse of the update takes a 1/N more.
-  constexpr float inv_n = 1.0f / N;
-  constexpr float inv_n2 = 1.0f / ((float)N * (float)N);
-  double acc[4] = {0.0, 0.0, 0.0, 0.0};
-  const float* iobs = a.iobs + (size_t)f * N * N;
-  float afar = MODE == kLsqmlFused ? a.a_far[slot] : 0.f;
-  // Each thread's 16 pixels (idx = tid + i·T): their counts and model intensity, read once.
-  constexpr int kPixPerThread = H * N / T;
-  float yo_r[kPixPerThread], ic_r[kPixPerThread];
+  // The field of a kStore pass, by the thread that reads it back.
+  float2* field = a.field + ((size_t)slot * C + r) * K * H * N + tid;
+#pragma unroll 1
+  for (int m = 0; m < K; ++m) {
+    if (MODE == kFromStore) {
 #pragma unroll
-  for (int i = 0; i < kPixPerThread; ++i) {
-    const int idx = tid + i * T;
-    const int c = idx % H, ky = idx / H;
-    yo_r[i] = iobs[ky * N + r * H + c];
-    float ic = 0.f;
-    for (int m = 0; m < K; ++m) ic += cnorm2(S[(m * H + c) * L + (ky ^ swz(m * H + c))]);
-    ic_r[i] = ic * inv_n2;
+      for (int i = 0; i < E; ++i) v[i] = field[(size_t)m * H * N + i * T];
+    } else if (MODE == kProjectKept) {
+      const float2* src = a.psi_out + ((size_t)slot * K + m) * plane + dpix;
+#pragma unroll
+      for (int i = 0; i < E; ++i) v[i] = src[i * kRow];
+    } else {
+      ln.columns_forward(v, m);
+    }
+    if ((MODE == kMlGrad || MODE == kBhGrad) && a.psi_out) {
+      float2* dst = a.psi_out + ((size_t)slot * K + m) * plane + dpix;
+#pragma unroll
+      for (int i = 0; i < E; ++i) dst[i * kRow] = v[i];
+    }
+    if (MODE == kStore) {
+#pragma unroll
+      for (int i = 0; i < E; ++i) field[(size_t)m * H * N + i * T] = v[i];
+    }
+#pragma unroll
+    for (int i = 0; i < E; ++i) ic[i] += fmaf(v[i].x, v[i].x, v[i].y * v[i].y);
+    // the last mode stays in registers
+    if (MODE != kStore && MODE != kLlk && m + 1 < K) ln.stash(v, m);
   }
+  if (from_field) __syncthreads();  // the twiddle table
+#pragma unroll
+  for (int i = 0; i < E; ++i) ic[i] *= inv_n2;
+  float afar = MODE == kLsqmlFused ? a.a_far[slot] : 0.f;
   if ((MODE == kStore || MODE == kFromStore) && a.cost == kCostPoisson && a.a_out) {
     // One pass of the Poisson xi solver over this frame: with prev the batch mean of the
     // previous pass, a = clip(prev/2 + Σ xi·(Ĩ − I/(1 − prev·xi)) / Σ xi²·Ĩ / 2, 0, 1).
@@ -367,74 +394,38 @@ __global__ void __launch_bounds__(FrameShape<N, C>::T,
                             : batch_mean(a.a_mid, a.frames, 0, a.nslot, red + 7);
     double num = 0.0, den = 0.0;
 #pragma unroll
-    for (int i = 0; i < kPixPerThread; ++i) {
-      const float yo = yo_r[i];
-      if (yo < 0.f) continue;
-      const double yp = (double)ic_r[i], yt = yo;
+    for (int i = 0; i < E; ++i) {
+      if (yo[i] < 0.f) continue;
+      const double yp = (double)ic[i], yt = yo[i];
       const double xi = 1.0 - yt / (yp + 1e-5);
       num += xi * (yp - yt / (1.0 - prev * xi));
       den += xi * xi * yp;
     }
-    cluster_sum2<N, C>(num, den, red, cluster);
+    cluster_sum2<T, C>(num, den, red, cluster);
     const double ratio = den > 0.0 ? num / den : 0.0;
     afar = (float)fmin(fmax(0.5 * prev + 0.5 * ratio, 0.0), 1.0);
     if (r == 0 && tid == 0) a.a_out[slot] = afar;
   }
+  if (MODE == kStore) {
+    if (a.icalc) {
 #pragma unroll
-  for (int i = 0; i < kPixPerThread; ++i) {
-    if (MODE == kStore && !a.icalc) break;
-    const int idx = tid + i * T;
-    const int c = idx % H, ky = idx / H;
-    const int kx = r * H + c;
-    const float ic = ic_r[i];
-    const float yo = yo_r[i];
-    const bool masked = yo < 0.f;
-    if (MODE == kStore) {
-      a.icalc[((size_t)slot * N + ky) * N + kx] = ic;
-      continue;
+      for (int i = 0; i < E; ++i) a.icalc[(size_t)slot * plane + dpix + i * kRow] = ic[i];
     }
-    if (MODE == kLlk || (MODE == kCarry && a.llk)) {
-      if (!masked) {
-        acc[0] += yo > 0.f ? (double)ic - yo + (double)yo * log((double)yo / ic) : (double)ic;
-        const double dg = (double)yo - ic;
-        acc[1] += dg * dg / ((double)yo + 1.0);
-        const double de = sqrt((double)yo) - sqrt((double)ic);
-        acc[2] += 4.0 * de * de;
-        acc[3] += ic;
-      }
-      if (MODE == kLlk) continue;
-    }
-    float fac;
-    if (MODE == kRpie) {
-      fac = masked ? 1.f : sqrtf(yo + 1e-7f) / (sqrtf(ic) + 1e-7f);
-    } else if (MODE == kProjectKept) {
-      // ApplyAmplitude (engine/ops.rs:83-107) minus the identity: the kept field Ψ = DFT(ψ)
-      // goes to ΔΨ = Ψ' − Ψ, whose inverse is the change ψ' − ψ itself (no model re-read)
-      fac = masked ? 0.f : sqrtf(yo) / fmaxf(sqrtf(ic), 1e-12f) - 1.f;
-    } else if (MODE == kProject || MODE == kCarry) {
-      // ApplyAmplitude (engine/ops.rs:83-107)
-      fac = masked ? 1.f : sqrtf(yo) / fmaxf(sqrtf(ic), 1e-12f);
-    } else if (MODE == kMlGrad) {
-      fac = masked ? 0.f : 2.f * (1.f - yo / fmaxf(ic, 1e-12f));
-    } else if (MODE == kBhGrad) {
-      // BH's residual (engine/bh.rs:255-265)
-      fac = masked ? 0.f : 2.f * (1.f - sqrtf(yo) / (sqrtf(ic) + 1e-8f));
-    } else {
-      float cres = 0.f;
-      if (!masked)
-        cres = a.cost == kCostPoisson ? 1.f - yo / (ic + 1e-6f)
-                                      : 2.f * (1.f - sqrtf(fmaxf(yo, 0.f)) / (sqrtf(ic) + 1e-9f));
-      fac = 1.f - afar * cres;
-    }
-    fac *= inv_n2;
-    for (int m = 0; m < K; ++m) {
-      float2& v = S[(m * H + c) * L + (ky ^ swz(m * H + c))];
-      v = cscale(v, fac);
-    }
+    return;
   }
-  (void)inv_n;
-
   if (MODE == kLlk || (MODE == kCarry && a.llk)) {
+    double acc[4] = {0.0, 0.0, 0.0, 0.0};
+#pragma unroll
+    for (int i = 0; i < E; ++i) {
+      if (yo[i] < 0.f) continue;
+      const double y = yo[i], c = ic[i];
+      acc[0] += yo[i] > 0.f ? c - y + y * log(y / c) : c;
+      const double dg = y - c;
+      acc[1] += dg * dg / (y + 1.0);
+      const double de = sqrt(y) - sqrt(c);
+      acc[2] += 4.0 * de * de;
+      acc[3] += c;
+    }
     block_sum<T>(acc, 4, red);
     csync<C>(cluster);
     if (r == 0 && tid == 0) {
@@ -447,72 +438,83 @@ __global__ void __launch_bounds__(FrameShape<N, C>::T,
     csync<C>(cluster);
     if (MODE == kLlk) return;
   }
-  if (MODE == kStore) {
-    __syncthreads();
-    float2* dst = a.field + ((size_t)slot * C + r) * K * H * N;
-#pragma unroll 8
-    for (int idx = tid; idx < K * H * N; idx += T) {
-      const int line = idx / N, e = idx % N;
-      dst[idx] = S[line * L + (e ^ swz(line))];
+  // The factor of every mode at the pixel, into ic.
+#pragma unroll
+  for (int i = 0; i < E; ++i) {
+    const float y = yo[i], c = ic[i];
+    const bool masked = y < 0.f;
+    float fac;
+    if (MODE == kRpie) {
+      fac = masked ? 1.f : sqrtf(y + 1e-7f) / (sqrtf(c) + 1e-7f);
+    } else if (MODE == kProjectKept) {
+      // ApplyAmplitude (engine/ops.rs:83-107) minus the identity: the kept field Ψ = DFT(ψ)
+      // goes to ΔΨ = Ψ' − Ψ, whose inverse is the change ψ' − ψ itself (no model re-read)
+      fac = masked ? 0.f : sqrtf(y) / fmaxf(sqrtf(c), 1e-12f) - 1.f;
+    } else if (MODE == kProject || MODE == kCarry) {
+      // ApplyAmplitude (engine/ops.rs:83-107)
+      fac = masked ? 1.f : sqrtf(y) / fmaxf(sqrtf(c), 1e-12f);
+    } else if (MODE == kMlGrad) {
+      fac = masked ? 0.f : 2.f * (1.f - y / fmaxf(c, 1e-12f));
+    } else if (MODE == kBhGrad) {
+      // BH's residual (engine/bh.rs:255-265)
+      fac = masked ? 0.f : 2.f * (1.f - sqrtf(y) / (sqrtf(c) + 1e-8f));
+    } else {
+      float cres = 0.f;
+      if (!masked)
+        cres = a.cost == kCostPoisson ? 1.f - y / (c + 1e-6f)
+                                      : 2.f * (1.f - sqrtf(fmaxf(y, 0.f)) / (sqrtf(c) + 1e-9f));
+      fac = 1.f - afar * cres;
     }
-    return;
+    ic[i] = fac * inv_n2;
   }
-  __syncthreads();
-  all_lines<N, C, +1>(S, K * H, ltw);
-  transpose<N, C>(S, K, cluster);
-  all_lines<N, C, +1>(S, K * H, ltw);
+#pragma unroll 1
+  for (int m = K - 1; m >= 0; --m) {
+    if (m + 1 < K) ln.unstash(v, m);
+#pragma unroll
+    for (int i = 0; i < E; ++i) v[i] = cscale_rn(v[i], ic[i]);
+    ln.columns_inverse(v, m);
+  }
+  L::publish();
 
-  // Epilogue on shifted rows: dst = ψ' − ψ (or ψ'), natural layout; the object window and the
-  // phase are read once per pixel.
-  auto epilogue = [&](float2* base, bool subtract) {
-    float2* dst = base + (size_t)slot * K * N * N;
-#pragma unroll 2
-    for (int idx = tid; idx < H * N; idx += T) {
-      const int yl = idx / N, jx = idx % N;
-      const int ny = (r * H + yl + N / 2) % N, nx = (jx + N / 2) % N;
-      float2 q = make_float2(0.f, 0.f);
-      if (subtract) q = a.quad[ny * N + nx];
-      for (int om = 0; om < a.nobj; ++om) {
-        float2 oq = make_float2(0.f, 0.f);
-        if (subtract)
-          oq = cmul(a.object[((size_t)om * a.nyo + corner.x + ny) * a.nxo + corner.y + nx], q);
-        for (int pm = 0; pm < a.nprobe; ++pm) {
-          const int m = om * a.nprobe + pm;
-          const int line = m * H + yl;
-          float2 v = S[line * L + (jx ^ swz(line))];
-          if (subtract)
-            v = csub(v, cmul(a.probe[(size_t)slot * a.probe_stride + ((size_t)pm * N + ny) * N + nx],
-                             oq));
-          dst[((size_t)m * N + ny) * N + nx] = v;
-        }
+  // Rows again, row-mapped: ψ' − ψ (or ψ'), natural layout.
+  constexpr bool subtract = MODE != kMlGrad && MODE != kBhGrad && MODE != kProjectKept;
+  float2 oq[E];
+  float unused = 0.f;
+#pragma unroll 1
+  for (int m = 0, om = 0, pm = 0; m < K; ++m) {
+    const size_t gi = ((size_t)slot * K + m) * plane + rpix;
+    ln.rows_inverse(v, m);
+    if (MODE == kCarry) {
+      // carried waves ← Π(S) + c_refl·(PO − S), in place (this thread read these pixels above)
+      if (a.c_refl != 0.f) {
+        if (pm == 0) window(oq, om, unused);
+        const float2* p = a.probe + (size_t)slot * a.probe_stride + pm * plane + rpix;
+        float2 po[E], x[E];
+#pragma unroll
+        for (int i = 0; i < E; ++i) x[i] = po[i] = cmul_rn(p[xof(i)], oq[i]);
+        carry_mix<N, C>(a, x, gi, false);
+#pragma unroll
+        for (int i = 0; i < E; ++i) v[i] = cadd(v[i], cscale(csub(po[i], x[i]), a.c_refl));
       }
-    }
-  };
-  if (MODE == kCarry) {
-    // carried waves ← Π(S) + c_refl·(PO − S), in place (this thread read these pixels above)
-#pragma unroll 2
-    for (int idx = tid; idx < H * N; idx += T) {
-      const int yl = idx / N, jx = idx % N;
-      const int ny = (r * H + yl + N / 2) % N, nx = (jx + N / 2) % N;
-      const int pix = ny * N + nx;
-      float2 oq = make_float2(0.f, 0.f);
-      if (a.c_refl != 0.f)
-        oq = cmul(a.object[(size_t)(corner.x + ny) * a.nxo + corner.y + nx], a.quad[pix]);
-      for (int m = 0; m < K; ++m) {
-        const int line = m * H + yl;
-        float2 v = S[line * L + (jx ^ swz(line))];
-        const size_t gi = ((size_t)slot * K + m) * N * N + pix;
-        if (a.c_refl != 0.f) {
-          const float2 po =
-              cmul(a.probe[(size_t)slot * a.probe_stride + (size_t)m * N * N + pix], oq);
-          v = cadd(v, cscale(csub(po, carry_mix<N>(a, po, slot, m, pix, K, false)), a.c_refl));
-        }
-        a.carry[gi] = v;
+      float2* dst = a.carry + gi;
+#pragma unroll
+      for (int i = 0; i < E; ++i) dst[xof(i)] = v[i];
+    } else {
+      if (subtract) {
+        if (pm == 0) window(oq, om, unused);
+        const float2* p = a.probe + (size_t)slot * a.probe_stride + pm * plane + rpix;
+#pragma unroll
+        for (int i = 0; i < E; ++i) v[i] = csub(v[i], cmul_rn(p[xof(i)], oq[i]));
       }
+      float2* dst = a.out + gi;
+#pragma unroll
+      for (int i = 0; i < E; ++i) dst[xof(i)] = v[i];
     }
-    return;
+    if (++pm == a.nprobe) {
+      pm = 0;
+      ++om;
+    }
   }
-  epilogue(a.out, MODE != kMlGrad && MODE != kBhGrad && MODE != kProjectKept);
 }
 
 }  // namespace ptyb

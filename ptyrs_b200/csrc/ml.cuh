@@ -29,7 +29,7 @@ struct GammaArgs {
   // Elements between consecutive slots' probe and probe direction: 0 for the shared ones,
   // K·N·N for the per-frame moved ones of the position model.
   int probe_stride;
-  // po = DFT(P·O·q) of every slot and mode as the gradient pass kept it, [slot][K][kx][ky],
+  // po = DFT(P·O·q) of every slot and mode as the gradient pass kept it, [slot][K][ky][kx],
   // and its exit-plane gradient field g = IDFT(2(1 − I/Ĩ)·po)/N² (masked 0), [slot][K][N][N].
   const float2* psi;
   const float2* g;
@@ -61,19 +61,12 @@ __global__ void __launch_bounds__(FrameShape<N, C>::T, 2) gamma_kernel(GammaArgs
   LineTwiddles<N> ltw;
   ltw.load(a.tw, tid % F::G);
   for (int i = tid; i < 3 * H * AS; i += T) acc[i] = 0.f;
-  // the kept detector columns the column phase reads, fetched into L2 now
-  for (int i = tid; i < K * H * (N / 16); i += T) {
-    const int row = i / (N / 16), m = row / H, c = row % H;
-    asm volatile("prefetch.global.L2 [%0];" ::"l"(a.psi + ((size_t)slot * K + m) * N * N +
-                                                  (size_t)(r * H + c) * N + (i % (N / 16)) * 16));
-  }
-
   // The b-term of den, Σ_pix 2·d·2·Re(p̄o·B)/N², by Parseval in the exit plane:
   // 2·Re Σ_x conj(g)·b with g = IDFT(2d·po)/N² the gradient pass's field (0 where masked).
   double gb = 0.0;
   for (int m = 0; m < K; ++m) {
     const int pm = m % a.nprobe, om = m / a.nprobe;
-    const float2* po_m = a.psi + ((size_t)slot * K + m) * N * N + (size_t)r * H * N;
+    const float2* po_m = a.psi + ((size_t)slot * K + m) * N * N + r * H;
     const float2* g_m = a.g + ((size_t)slot * K + m) * N * N;
     // Exit-plane rows of a; b and its product with g on the way.
 #pragma unroll 4
@@ -95,8 +88,8 @@ __global__ void __launch_bounds__(FrameShape<N, C>::T, 2) gamma_kernel(GammaArgs
     // Columns kx = r·H + c, elements ky; po read from the gradient pass's columns.
 #pragma unroll 4
     for (int idx = tid; idx < H * N; idx += T) {
-      const int c = idx / N, ky = idx % N;
-      const float2 po = po_m[(size_t)c * N + ky], v = S1[c * L + (ky ^ swz(c))];
+      const int c = idx % H, ky = idx / H;
+      const float2 po = po_m[(size_t)ky * N + c], v = S1[c * L + (ky ^ swz(c))];
       acc[c * AS + ky] += cnorm2(po) * inv_n2;
       acc[(H + c) * AS + ky] += (po.x * v.x + po.y * v.y) * inv_n2;
       acc[(2 * H + c) * AS + ky] += cnorm2(v) * inv_n2;

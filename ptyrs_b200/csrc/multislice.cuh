@@ -211,7 +211,7 @@ __global__ void __launch_bounds__(FrameShape<N, C>::T, frame_min_blocks<N, C>())
       num += xi * (yp - yt / (1.0 - prev * xi));
       den += xi * xi * yp;
     }
-    cluster_sum2<N, C>(num, den, red, cluster);
+    cluster_sum2<T, C>(num, den, red, cluster);
     const double ratio = den > 0.0 ? num / den : 0.0;
     afar = (float)fmin(fmax(0.5 * prev + 0.5 * ratio, 0.0), 1.0);
     if (r == 0 && tid == 0) a.a_out[slot] = afar;

@@ -201,7 +201,7 @@ __global__ void __launch_bounds__(FrameShape<N, C>::T,
       }
       __syncthreads();  // the next mode's spectrum overwrites the planes read above
     }
-    cluster_sum4<N, C>(v4, red, cluster);
+    cluster_sum4<T, C>(v4, red, cluster);
     if (r == 0 && tid == 0)
 #pragma unroll
       for (int k = 0; k < 4; ++k) a.sums[(size_t)f * 4 + k] = v4[k];

@@ -6,9 +6,9 @@
 
 namespace ptyb {
 
-// One launch of `kern` over nslot clusters of C CTAs with `smem` bytes of dynamic shared memory
+// One launch of `kern` over nslot clusters of C CTAs of T threads with `smem` bytes of dynamic shared memory
 // each; with `occupancy`, cudaErrorLaunchOutOfResources when no cluster of that shape fits.
-template <int N, int C, typename Kern, typename Args>
+template <int N, int C, int T = FrameShape<N, C>::T, typename Kern, typename Args>
 cudaError_t launch_clusters(Kern kern, const Args& a, int nslot, size_t smem, cudaStream_t s,
                             bool occupancy = false) {
   cudaError_t e =
@@ -20,7 +20,7 @@ cudaError_t launch_clusters(Kern kern, const Args& a, int nslot, size_t smem, cu
   }
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3(nslot * C);
-  cfg.blockDim = dim3(FrameShape<N, C>::T);
+  cfg.blockDim = dim3(T);
   cfg.dynamicSmemBytes = smem;
   cfg.stream = s;
   cudaLaunchAttribute attr[1];
@@ -41,20 +41,21 @@ cudaError_t launch_clusters(Kern kern, const Args& a, int nslot, size_t smem, cu
 
 template <int N, int C>
 cudaError_t frame_modes(int mode, const FrameArgs& a, int nslot, int K, cudaStream_t s) {
+  constexpr int T = PlaneShape<N, C>::T;
   const size_t smem = frame_smem_bytes<N, C>(K);
   switch (mode) {
-    case kRpie: return launch_clusters<N, C>(frame_kernel<N, C, kRpie>, a, nslot, smem, s);
+    case kRpie: return launch_clusters<N, C, T>(frame_kernel<N, C, kRpie>, a, nslot, smem, s);
     case kLsqmlFused:
-      return launch_clusters<N, C>(frame_kernel<N, C, kLsqmlFused>, a, nslot, smem, s);
-    case kMlGrad: return launch_clusters<N, C>(frame_kernel<N, C, kMlGrad>, a, nslot, smem, s);
-    case kBhGrad: return launch_clusters<N, C>(frame_kernel<N, C, kBhGrad>, a, nslot, smem, s);
-    case kLlk: return launch_clusters<N, C>(frame_kernel<N, C, kLlk>, a, nslot, smem, s);
-    case kStore: return launch_clusters<N, C>(frame_kernel<N, C, kStore>, a, nslot, smem, s);
+      return launch_clusters<N, C, T>(frame_kernel<N, C, kLsqmlFused>, a, nslot, smem, s);
+    case kMlGrad: return launch_clusters<N, C, T>(frame_kernel<N, C, kMlGrad>, a, nslot, smem, s);
+    case kBhGrad: return launch_clusters<N, C, T>(frame_kernel<N, C, kBhGrad>, a, nslot, smem, s);
+    case kLlk: return launch_clusters<N, C, T>(frame_kernel<N, C, kLlk>, a, nslot, smem, s);
+    case kStore: return launch_clusters<N, C, T>(frame_kernel<N, C, kStore>, a, nslot, smem, s);
     case kFromStore:
-      return launch_clusters<N, C>(frame_kernel<N, C, kFromStore>, a, nslot, smem, s);
+      return launch_clusters<N, C, T>(frame_kernel<N, C, kFromStore>, a, nslot, smem, s);
     case kProjectKept:
-      return launch_clusters<N, C>(frame_kernel<N, C, kProjectKept>, a, nslot, smem, s);
-    case kCarry: return launch_clusters<N, C>(frame_kernel<N, C, kCarry>, a, nslot, smem, s);
+      return launch_clusters<N, C, T>(frame_kernel<N, C, kProjectKept>, a, nslot, smem, s);
+    case kCarry: return launch_clusters<N, C, T>(frame_kernel<N, C, kCarry>, a, nslot, smem, s);
   }
   return cudaErrorInvalidValue;
 }
