@@ -49,22 +49,30 @@ struct MoveArgs {
 // numpy fftfreq of index k of n points (engine/features.rs:337-344).
 PTYB_D float fft_freq(int k, int n) { return (float)(k < (n + 1) / 2 ? k : k - n) / (float)n; }
 
+// Shared memory of K planes: frame_smem_bytes and the translation phase's N row factors.
+template <int N, int C>
+__host__ __device__ constexpr size_t move_smem_bytes(int K) {
+  return frame_smem_bytes<N, C>(K) + N * sizeof(float2);
+}
+
+// One frame per cluster, planes through plane.cuh's line transforms: forward from natural rows
+// (or a spectrum read in the columns), the phase in the columns, inverse to natural rows. As the
+// frame kernel, bound by latency (its exchanges and cluster barriers); per frame on one B200 at
+// 256² x 2 modes: moves from the spectrum 1.42 -> 0.93 us, probe gradient spectra 1.57 -> 1.03,
+// position sums 3.21 -> 2.21 (four inverse transforms), one plane's spectrum 27 -> 16 us a call.
 template <int N, int C, int MODE>
-__global__ void __launch_bounds__(FrameShape<N, C>::T,
-                                  N == 256 && FrameShape<N, C>::T <= 256 &&
-                                          (MODE == kFromSpectrum || MODE == kBackSpectrum ||
-                                           MODE == kSpectrum || MODE == kPlainInverse)
-                                      ? 3
-                                      : frame_min_blocks<N, C>())
+__global__ void __launch_bounds__(PlaneShape<N, C>::T, plane_min_blocks<N, C>())
     move_kernel(MoveArgs a) {
-  using F = FrameShape<N, C>;
-  constexpr int H = F::H, T = F::T, L = F::L;
-  extern __shared__ __align__(16) unsigned char smem_raw[];
+  using L = Lines<N, C>;
+  constexpr int H = L::H, T = L::T, E = L::N1, N2 = L::N2;
+  extern __shared__ __align__(128) unsigned char plane_smem[];
   const int K = MODE == kDerivWindow ? 2 : a.K;
   // planes held in shared memory: the position sums hold the two axes of one mode at a time
   const int KP = MODE == kDerivSums ? max(K, 2) : K;
-  float2* S = reinterpret_cast<float2*>(smem_raw);
-  double* red = reinterpret_cast<double*>(S + (size_t)KP * H * L + N);
+  float2* S = reinterpret_cast<float2*>(plane_smem);
+  float2* table = S + (size_t)KP * H * N;
+  float2* ey = table + N;
+  double* red = reinterpret_cast<double*>(ey + N);
   cg::cluster_group cluster = cg::this_cluster();
   const int r = C > 1 ? (int)cluster.block_rank() : 0;
   const int slot = blockIdx.x / C;
@@ -72,134 +80,128 @@ __global__ void __launch_bounds__(FrameShape<N, C>::T,
   const int f = one ? 0 : a.frames[slot];
   const int2 corner = one ? make_int2(0, 0) : a.corners[f];
   const int tid = threadIdx.x;
-  LineTwiddles<N> ltw;
-  ltw.load(a.tw, tid % F::G);
-  const size_t plane = (size_t)N * N;
-  float2* out = a.planes + (size_t)slot * K * plane;
+  const L ln(S, table, r);
+  L::fill_table(table, a.tw);
+  constexpr size_t plane = (size_t)N * N;
   constexpr float inv_n2 = 1.0f / ((float)N * (float)N);
+  constexpr float two_pi = 2.f * 3.14159265358979f;
   constexpr bool from_spec = MODE == kFromSpectrum || MODE == kDerivSums ||
-                              MODE == kPlainInverse || MODE == kDerivMove;
+                             MODE == kPlainInverse || MODE == kDerivMove;
   constexpr bool in_place = MODE == kMoveBack || MODE == kMoveOwn;
   constexpr bool moves = in_place || MODE == kFromSpectrum || MODE == kDerivSums ||
-                         MODE == kDerivMove ||
-                         MODE == kBackSpectrum;
-  constexpr bool bare = MODE == kDerivWindow;
+                         MODE == kDerivMove || MODE == kBackSpectrum;
+  constexpr int kRow = N2 * N;  // pixels between a thread's elements of a column
+  // Row-mapped: natural row y, first element's pixel; column-mapped: column kx, its first ky's.
+  const int y = r * H + ln.y, rpix = y * N + ln.rt;
+  const int kx = r * H + ln.c, cpix = ln.t * N + kx;
+  float2* out = a.planes + (size_t)slot * K * plane;
+  const float2* obj = a.object + (size_t)(corner.x + y) * a.nxo + corner.y + ln.rt;
+  const float2* quad = a.quad + rpix;
 
-  float dy = 0.f, dx = 0.f;
-  if (moves) {
-    const float sgn = MODE == kMoveBack || MODE == kBackSpectrum ? -1.f : 1.f;
-    dy = sgn * (float)a.offsets[2 * f];
-    dx = sgn * (float)a.offsets[2 * f + 1];
-  }
   // The translation phase exp(−2πi f·d) = exp(−2πi fy·dy)·exp(−2πi fx·dx), over N²: the row
-  // factor for every ky in the free N-entry region after the planes, the column factor of this
-  // thread's one column (T is a multiple of H, so a thread keeps c = tid % H).
-  float2* ey = S + (size_t)KP * H * L;
+  // factor of every ky in shared memory, the column factor of this thread's one column.
   float2 ex = make_float2(1.f, 0.f);
   if (moves) {
+    const float sgn = MODE == kMoveBack || MODE == kBackSpectrum ? -1.f : 1.f;
+    const float dy = sgn * (float)a.offsets[2 * f], dx = sgn * (float)a.offsets[2 * f + 1];
+    float sn, cs;
     for (int k = tid; k < N; k += T) {
-      float sn, cs;
       sincospif(-2.f * fft_freq(k, N) * dy, &sn, &cs);
       ey[k] = make_float2(cs * inv_n2, sn * inv_n2);
     }
-    float sn, cs;
-    sincospif(-2.f * fft_freq(r * H + tid % H, N) * dx, &sn, &cs);
+    sincospif(-2.f * fft_freq(kx, N) * dx, &sn, &cs);
     ex = make_float2(cs, sn);
   }
+  // The phase at element i of this thread's column (fy of it beside).
+  auto phase = [&](int i) { return moves ? cmul(ey[N2 * i + ln.t], ex) : make_float2(1.f, 0.f); };
+  auto freq_y = [&](int i) { return two_pi * fft_freq(N2 * i + ln.t, N); };
+  const float freq_x = two_pi * fft_freq(kx, N);
 
+  float2 v[E];
   if (!from_spec) {
-    // Natural-layout rows r·H .. r·H+H-1 of every plane, then the forward transform.
-#pragma unroll 2
-    for (int idx = tid; idx < H * N; idx += T) {
-      const int yl = idx / N, x = idx % N, y = r * H + yl;
-      float2 w;
-      if (MODE == kSpectrum || in_place)
-        w = a.quad[y * N + x];
-      else if (MODE == kBackSpectrum)
-        w = cconj(a.object[(size_t)(corner.x + y) * a.nxo + corner.y + x]);
-      for (int m = 0; m < K; ++m) {
-        float2 v;
-        if (MODE == kSpectrum)
-          v = cmul(w, a.probe[m * plane + y * N + x]);
-        else if (in_place)
-          v = cmul(w, out[m * plane + y * N + x]);
-        else if (MODE == kBackSpectrum) {
-          float2 cv = a.c[(size_t)slot * K * plane + m * plane + y * N + x];
-          if (a.minus)
-            cv = csub(cv, cmul(cmul(a.minus[(size_t)slot * K * plane + m * plane + y * N + x],
-                                    cconj(w)),
-                               a.quad[y * N + x]));
-          v = cmul(w, cv);
+    // Natural-layout rows, times q or the window's conjugate, through the row transforms; the
+    // window derivatives transform their one plane once for both axes.
+    float2 w[E];
+    if (MODE != kDerivWindow) {
+      const float2* src = MODE == kBackSpectrum ? obj : quad;
+#pragma unroll
+      for (int i = 0; i < E; ++i) w[i] = src[N2 * i];
+    }
+    const int kin = MODE == kDerivWindow ? 1 : K;
+#pragma unroll 1
+    for (int m = 0; m < kin; ++m) {
+      const float2* src = MODE == kDerivWindow    ? obj
+                          : MODE == kSpectrum     ? a.probe + m * plane + rpix
+                          : MODE == kBackSpectrum ? a.c + ((size_t)slot * K + m) * plane + rpix
+                                                  : out + m * plane + rpix;
+#pragma unroll
+      for (int i = 0; i < E; ++i) v[i] = src[N2 * i];
+      if (MODE == kBackSpectrum) {
+        if (a.minus) {
+          const float2* wave = a.minus + ((size_t)slot * K + m) * plane + rpix;
+#pragma unroll
+          for (int i = 0; i < E; ++i)
+            v[i] = csub(v[i], cmul(cmul(wave[N2 * i], w[i]), quad[N2 * i]));
         }
-        else
-          v = a.object[(size_t)(corner.x + y) * a.nxo + corner.y + x];
-        const int line = m * H + yl;
-        S[line * L + (x ^ swz(line))] = v;
+#pragma unroll
+        for (int i = 0; i < E; ++i) v[i] = cmulc(w[i], v[i]);
+      } else if (MODE != kDerivWindow) {
+#pragma unroll
+        for (int i = 0; i < E; ++i) v[i] = cmul(w[i], v[i]);
       }
+      if (m == 0) __syncthreads();  // the twiddle table, the row factors
+      ln.rows_forward(v, m);
     }
-    __syncthreads();
-    all_lines<N, C, -1>(S, K * H, ltw);
-    transpose<N, C>(S, K, cluster);
-    all_lines<N, C, -1>(S, K * H, ltw);
-    if (MODE == kSpectrum || MODE == kBackSpectrum) {
-      // Spectrum columns kx = r·H + c (lines m·H + c, elements ky) to [slot][m][ky][kx].
-#pragma unroll 2
-      for (int idx = tid; idx < H * N; idx += T) {
-        const int c = idx % H, ky = idx / H;
-        const float2 e = MODE == kBackSpectrum ? cmul(ey[ky], ex) : make_float2(1.f, 0.f);
-        for (int m = 0; m < K; ++m)
-          out[((size_t)m * N + ky) * N + r * H + c] =
-              cmul(S[(m * H + c) * L + (ky ^ swz(m * H + c))], e);
-      }
-      return;
-    }
-  } else if (moves) {
-    __syncthreads();  // the row factors
+    L::publish();
   }
 
   if (MODE == kDerivSums) {
-    // Both axes of one mode at a time, the planes holding ∂_y and ∂_x of mode m's moved probe:
-    // each mode's spectrum, field plane and window are read once for both axes.
-    constexpr float two_pi = 2.f * 3.14159265358979f;
-    const float2* cf = a.c + (size_t)slot * K * plane;
+    // Both axes of one mode at a time, the planes holding ∂_y and ∂_x of mode m's moved probe;
+    // the field plane and the window are read per axis, the second time from the caches (held
+    // in registers over the second axis' transform they spilled).
+    const float2* cf = a.c + (size_t)slot * K * plane + rpix;
     double v4[4] = {0.0, 0.0, 0.0, 0.0};  // num_y, num_x, den_y, den_x
 #pragma unroll 1
     for (int m = 0; m < K; ++m) {
-#pragma unroll 2
-      for (int idx = tid; idx < H * N; idx += T) {
-        const int c = idx % H, ky = idx / H, kx = r * H + c;
-        const float2 v = cmul(a.spec[((size_t)m * N + ky) * N + kx], cmul(ey[ky], ex));
-        // × (−2πi·f_axis): the derivative of the translation phase (engine/features.rs:372-387)
-        const float wy = two_pi * fft_freq(ky, N), wx = two_pi * fft_freq(kx, N);
-        S[c * L + (ky ^ swz(c))] = make_float2(wy * v.y, -wy * v.x);
-        S[(H + c) * L + (ky ^ swz(H + c))] = make_float2(wx * v.y, -wx * v.x);
+      float2 s[E];
+      const float2* spec = a.spec + m * plane + cpix;
+#pragma unroll
+      for (int i = 0; i < E; ++i) s[i] = spec[i * kRow];
+      if (m == 0) __syncthreads();  // the twiddle table, the row factors
+#pragma unroll
+      for (int i = 0; i < E; ++i) s[i] = cmul(s[i], phase(i));
+      // × (−2πi·f_axis): the derivative of the translation phase (engine/features.rs:372-387)
+#pragma unroll
+      for (int i = 0; i < E; ++i) {
+        const float w = freq_y(i);
+        v[i] = make_float2(w * s[i].y, -w * s[i].x);
       }
-      __syncthreads();
-      // two planes, as a value the compiler does not unroll the transforms' plane loops over
-      int two = 2;
-      asm volatile("" : "+r"(two));
-      all_lines<N, C, +1>(S, two * H, ltw);
-      transpose<N, C>(S, two, cluster);
-      all_lines<N, C, +1>(S, two * H, ltw);
+      ln.columns_inverse(v, 0);
+#pragma unroll
+      for (int i = 0; i < E; ++i) v[i] = make_float2(freq_x * s[i].y, -freq_x * s[i].x);
+      ln.columns_inverse(v, 1);
+      L::publish();
       // dψ = O·∂W on natural rows; num = Σ Re(conj(c)·dψ), den = Σ |dψ|² over modes and
       // pixels (engine/features.rs:992-1025)
-#pragma unroll 2
-      for (int idx = tid; idx < H * N; idx += T) {
-        const int yl = idx / N, x = idx % N, y = r * H + yl;
-        const float2 o = a.object[(size_t)(corner.x + y) * a.nxo + corner.y + x];
-        float2 v = cf[m * plane + y * N + x];
-        if (a.minus)
-          v = csub(v, cmul(cmul(a.minus[(size_t)slot * K * plane + m * plane + y * N + x], o),
-                           a.quad[y * N + x]));
 #pragma unroll
-        for (int ax = 0; ax < 2; ++ax) {
-          const int line = ax * H + yl;
-          const float2 d = cmul(o, S[line * L + (x ^ swz(line))]);
-          v4[ax] += (double)v.x * d.x + (double)v.y * d.y;
+      for (int ax = 0; ax < 2; ++ax) {
+        ln.rows_inverse(v, ax);
+        float2 cv[E];
+#pragma unroll
+        for (int i = 0; i < E; ++i) cv[i] = cf[m * plane + N2 * i];
+        if (a.minus) {
+          const float2* wave = a.minus + ((size_t)slot * K + m) * plane + rpix;
+#pragma unroll
+          for (int i = 0; i < E; ++i)
+            cv[i] = csub(cv[i], cmul(cmul(wave[N2 * i], obj[N2 * i]), quad[N2 * i]));
+        }
+#pragma unroll
+        for (int i = 0; i < E; ++i) {
+          const float2 d = cmul(obj[N2 * i], v[i]);
+          v4[ax] += (double)cv[i].x * d.x + (double)cv[i].y * d.y;
           v4[2 + ax] += (double)d.x * d.x + (double)d.y * d.y;
         }
       }
-      __syncthreads();  // the next mode's spectrum overwrites the planes read above
     }
     cluster_sum4<T, C>(v4, red, cluster);
     if (r == 0 && tid == 0)
@@ -208,18 +210,36 @@ __global__ void __launch_bounds__(FrameShape<N, C>::T,
     return;
   }
 
-  {
-    // Spectrum: column kx = r·H + c as line (m·H + c), element ky.
-#pragma unroll 2
-    for (int idx = tid; idx < H * N; idx += T) {
-      const int c = idx % H, ky = idx / H, kx = r * H + c;
-      const float fy = fft_freq(ky, N), fx = fft_freq(kx, N);
-      float2 e = make_float2(1.f, 0.f);
-      if (moves) {
-        e = cmul(ey[ky], ex);
-        if (MODE == kDerivMove) {
-          // × (−2πi·f_a) or × (−2πi·f_a)(−2πi·f_b) = −4π²·f_a·f_b
-          const float wy = 2.f * 3.14159265358979f * fy, wx = 2.f * 3.14159265358979f * fx;
+  if (MODE == kDerivWindow) {
+    // × 2πi·f_axis / N² for both axes
+    ln.columns_forward(v, 0);
+    float2 u[E];
+#pragma unroll
+    for (int ax = 0; ax < 2; ++ax) {
+#pragma unroll
+      for (int i = 0; i < E; ++i) {
+        const float w = (ax == 0 ? freq_y(i) : freq_x) * inv_n2;
+        u[i] = make_float2(-w * v[i].y, w * v[i].x);
+      }
+      ln.columns_inverse(u, ax);
+    }
+  } else {
+#pragma unroll 1
+    for (int m = 0; m < K; ++m) {
+      if (from_spec) {
+        const float2* spec = a.spec + m * plane + cpix;
+#pragma unroll
+        for (int i = 0; i < E; ++i) v[i] = spec[i * kRow];
+        if (m == 0) __syncthreads();  // the twiddle table, the row factors
+      } else {
+        ln.columns_forward(v, m);
+      }
+      if (MODE == kDerivMove) {
+        // × (−2πi·f_a) or × (−2πi·f_a)(−2πi·f_b) = −4π²·f_a·f_b
+#pragma unroll
+        for (int i = 0; i < E; ++i) {
+          float2 e = phase(i);
+          const float wy = freq_y(i), wx = freq_x;
           if (a.deriv <= 2) {
             const float w = a.deriv == 1 ? wy : wx;
             e = make_float2(w * e.y, -w * e.x);
@@ -227,41 +247,37 @@ __global__ void __launch_bounds__(FrameShape<N, C>::T,
             const float w = a.deriv == 3 ? -wy * wy : a.deriv == 4 ? -wy * wx : -wx * wx;
             e = make_float2(w * e.x, w * e.y);
           }
+          v[i] = cmul(v[i], e);
         }
+      } else if (moves) {
+#pragma unroll
+        for (int i = 0; i < E; ++i) v[i] = cmul(v[i], phase(i));
       }
-      for (int m = 0; m < K; ++m) {
-        float2& v = S[(m * H + c) * L + (ky ^ swz(m * H + c))];
-        if (from_spec) {
-          v = cmul(a.spec[((size_t)m * N + ky) * N + kx], e);
-        } else if (MODE == kDerivWindow) {
-          const float w = 2.f * 3.14159265358979f * (m == 0 ? fy : fx) * inv_n2;
-          v = make_float2(-w * v.y, w * v.x);  // × 2πi·f_axis
-        } else {
-          v = cmul(v, e);
-        }
-      }
-    }
-    __syncthreads();
-    all_lines<N, C, +1>(S, K * H, ltw);
-    transpose<N, C>(S, K, cluster);
-    all_lines<N, C, +1>(S, K * H, ltw);
-
-#pragma unroll 2
-    for (int idx = tid; idx < H * N; idx += T) {
-      const int yl = idx / N, x = idx % N, y = r * H + yl;
-      const float2 cq = bare ? make_float2(1.f, 0.f) : cconj(a.quad[y * N + x]);
-      for (int m = 0; m < K; ++m) {
-        const int line = m * H + yl;
-        const float2 v = S[line * L + (x ^ swz(line))];
-        out[m * plane + y * N + x] = bare ? v : cmul(cq, v);
+      if (MODE == kSpectrum || MODE == kBackSpectrum) {
+        // the spectrum's columns to [slot][m][ky][kx]
+        float2* dst = out + m * plane + cpix;
+#pragma unroll
+        for (int i = 0; i < E; ++i) dst[i * kRow] = v[i];
+      } else {
+        ln.columns_inverse(v, m);
       }
     }
   }
-}
+  if (MODE == kSpectrum || MODE == kBackSpectrum) return;
+  L::publish();
 
-template <int N, int C>
-__host__ __device__ constexpr size_t move_smem_bytes(int K) {
-  return frame_smem_bytes<N, C>(K);
+  float2 w[E];
+  if (MODE != kDerivWindow) {
+#pragma unroll
+    for (int i = 0; i < E; ++i) w[i] = quad[N2 * i];
+  }
+#pragma unroll 1
+  for (int m = 0; m < K; ++m) {
+    ln.rows_inverse(v, m);
+    float2* dst = out + m * plane + rpix;
+#pragma unroll
+    for (int i = 0; i < E; ++i) dst[N2 * i] = MODE == kDerivWindow ? v[i] : cmulc(w[i], v[i]);
+  }
 }
 
 // planes[slot][m] = w·χ_m per natural pixel: each frame's probe direction before its adjoint

@@ -62,23 +62,24 @@ cudaError_t frame_modes(int mode, const FrameArgs& a, int nslot, int K, cudaStre
 
 template <int N, int C>
 cudaError_t move_modes(int mode, const MoveArgs& a, int nslot, int K, cudaStream_t s) {
+  constexpr int T = PlaneShape<N, C>::T;
   const size_t smem = move_smem_bytes<N, C>(K);
   switch (mode) {
-    case kMoveBack: return launch_clusters<N, C>(move_kernel<N, C, kMoveBack>, a, nslot, smem, s);
+    case kMoveBack: return launch_clusters<N, C, T>(move_kernel<N, C, kMoveBack>, a, nslot, smem, s);
     case kDerivWindow:
-      return launch_clusters<N, C>(move_kernel<N, C, kDerivWindow>, a, nslot, smem, s);
-    case kSpectrum: return launch_clusters<N, C>(move_kernel<N, C, kSpectrum>, a, nslot, smem, s);
+      return launch_clusters<N, C, T>(move_kernel<N, C, kDerivWindow>, a, nslot, smem, s);
+    case kSpectrum: return launch_clusters<N, C, T>(move_kernel<N, C, kSpectrum>, a, nslot, smem, s);
     case kFromSpectrum:
-      return launch_clusters<N, C>(move_kernel<N, C, kFromSpectrum>, a, nslot, smem, s);
+      return launch_clusters<N, C, T>(move_kernel<N, C, kFromSpectrum>, a, nslot, smem, s);
     case kDerivSums:
-      return launch_clusters<N, C>(move_kernel<N, C, kDerivSums>, a, nslot, smem, s);
+      return launch_clusters<N, C, T>(move_kernel<N, C, kDerivSums>, a, nslot, smem, s);
     case kBackSpectrum:
-      return launch_clusters<N, C>(move_kernel<N, C, kBackSpectrum>, a, nslot, smem, s);
+      return launch_clusters<N, C, T>(move_kernel<N, C, kBackSpectrum>, a, nslot, smem, s);
     case kPlainInverse:
-      return launch_clusters<N, C>(move_kernel<N, C, kPlainInverse>, a, nslot, smem, s);
-    case kMoveOwn: return launch_clusters<N, C>(move_kernel<N, C, kMoveOwn>, a, nslot, smem, s);
+      return launch_clusters<N, C, T>(move_kernel<N, C, kPlainInverse>, a, nslot, smem, s);
+    case kMoveOwn: return launch_clusters<N, C, T>(move_kernel<N, C, kMoveOwn>, a, nslot, smem, s);
     case kDerivMove:
-      return launch_clusters<N, C>(move_kernel<N, C, kDerivMove>, a, nslot, smem, s);
+      return launch_clusters<N, C, T>(move_kernel<N, C, kDerivMove>, a, nslot, smem, s);
   }
   return cudaErrorInvalidValue;
 }
