@@ -141,7 +141,8 @@ cudaError_t SideKernels<N>::slice(int C, int mode, const SliceArgs& a, int nslot
 template <int N>
 cudaError_t SideKernels<N>::gamma(const GammaArgs& a, int nslot, cudaStream_t s) {
   constexpr int C = gamma_cluster(N);
-  return launch_clusters<N, C>(gamma_kernel<N, C>, a, nslot, gamma_smem_bytes<N, C>(), s, true);
+  return launch_clusters<N, C, PlaneShape<N, C>::T>(
+      gamma_kernel<N, C>, a, nslot, frame_smem_bytes<N, C>(a.nprobe * a.nobj), s, true);
 }
 
 template <int N>
