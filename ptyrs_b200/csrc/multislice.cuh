@@ -7,7 +7,9 @@
 // them and the next slice's window (the last also the exit phase q), each incident wave stored
 // for the gathers; then the far-field FFT, the xi solver's first pass and the detector field.
 // Backward: the field, the second xi pass, the residual, the inverse FFT and χ of the last
-// slice, then per gap back through conj(q·O) and the conjugate transfer function.
+// slice, then per gap back through conj(q·O) and the conjugate transfer function. The lines stay
+// in registers between the transposes (plane.cuh); per frame of 128² x 2 through three slices on
+// one B200: forward 1.96 -> 1.04 us, backward 2.65 -> 1.21 us.
 #pragma once
 #include "frame.cuh"
 
@@ -27,31 +29,6 @@ struct SliceArgs {
 // back-propagation through the slices into `chi` (no subtraction): every slice's 2·∂L/∂ψ_s*,
 // the adjoint of the multislice model.
 enum SliceMode : int { kSliceForward = 0, kSliceBackward = 1, kSliceLlk = 2, kSliceGrad = 3 };
-
-// Window of slice s times `v` for every plane's rows of this CTA (shifted layout); the last
-// slice also takes q. `conj_mode` multiplies by conj(q·O) instead.
-template <int N, int C>
-PTYB_D void apply_window(float2* S, const SliceArgs& a, int s, int2 corner, int r, int K,
-                         bool conj_mode) {
-  using F = FrameShape<N, C>;
-  constexpr int H = F::H, T = F::T, L = F::L;
-  const bool last = s + 1 == a.nslice;
-  const float2* obj = a.f.object + (size_t)s * a.obj_plane;
-#pragma unroll 2
-  for (int idx = threadIdx.x; idx < H * N; idx += T) {
-    const int yl = idx / N, jx = idx % N;
-    const int ny = (r * H + yl + N / 2) % N, nx = (jx + N / 2) % N;
-    float2 w = obj[(size_t)(corner.x + ny) * a.f.nxo + corner.y + nx];
-    if (last) w = cmul(w, a.f.quad[ny * N + nx]);
-    if (conj_mode) w = cconj(w);
-    for (int m = 0; m < K; ++m) {
-      const int line = m * H + yl;
-      float2& v = S[line * L + (jx ^ swz(line))];
-      v = cmul(v, w);
-    }
-  }
-  __syncthreads();
-}
 
 // The planes through gap s in place: FFT, × tf (or its conjugate) / N², inverse FFT.
 template <int N, int C>
@@ -80,109 +57,142 @@ PTYB_D void through_gap(float2* S, const float2* tf, int K, bool adjoint, const 
   all_lines<N, C, +1>(S, K * H, ltw);
 }
 
-// This CTA's rows of every plane to `dst` ([K][N][N] natural layout), or loaded from it.
-template <int N, int C>
-PTYB_D void rows_io(float2* S, float2* dst, int r, int K, bool store) {
-  using F = FrameShape<N, C>;
-  constexpr int H = F::H, T = F::T, L = F::L;
-#pragma unroll 2
-  for (int idx = threadIdx.x; idx < H * N; idx += T) {
-    const int yl = idx / N, jx = idx % N;
-    const int ny = (r * H + yl + N / 2) % N, nx = (jx + N / 2) % N;
-    for (int m = 0; m < K; ++m) {
-      const int line = m * H + yl;
-      float2& v = S[line * L + (jx ^ swz(line))];
-      float2* g = dst + ((size_t)m * N + ny) * N + nx;
-      if (store)
-        *g = v;
-      else
-        v = *g;
-    }
-  }
-  __syncthreads();
-}
-
 template <int N, int C, int MODE>
-__global__ void __launch_bounds__(FrameShape<N, C>::T, frame_min_blocks<N, C>())
+__global__ void __launch_bounds__(PlaneShape<N, C>::T, plane_min_blocks<N, C>())
     slice_kernel(SliceArgs sa) {
-  using F = FrameShape<N, C>;
-  constexpr int H = F::H, T = F::T, L = F::L;
+  using L = Lines<N, C>;
+  constexpr int H = L::H, T = L::T, E = L::N1, N2 = L::N2;
   const FrameArgs& a = sa.f;
-  extern __shared__ __align__(16) unsigned char smem_raw[];
+  extern __shared__ __align__(128) unsigned char plane_smem[];
   const int K = a.nprobe;
-  float2* S = reinterpret_cast<float2*>(smem_raw);
-  float2* twb = S + (size_t)K * H * L;
-  double* red = reinterpret_cast<double*>(twb + N);
+  float2* S = reinterpret_cast<float2*>(plane_smem);
+  float2* table = S + (size_t)K * H * N;
+  double* red = reinterpret_cast<double*>(table + N);
   cg::cluster_group cluster = cg::this_cluster();
   const int r = C > 1 ? (int)cluster.block_rank() : 0;
   const int slot = blockIdx.x / C;
   const int f = a.frames[slot];
   const int2 corner = a.corners[f];
   const int tid = threadIdx.x;
-  LineTwiddles<N> ltw;
-  ltw.load(a.tw, tid % F::G);
-  const size_t frame_planes = (size_t)K * N * N;
+  const L ln(S, table, r);
+  L::fill_table(table, a.tw);
+  constexpr size_t plane = (size_t)N * N;
+  const size_t frame_planes = (size_t)K * plane;
   const size_t slice_stride = (size_t)a.nslot * frame_planes;  // one slice's [slot][K][N][N]
   constexpr float inv_n2 = 1.0f / ((float)N * (float)N);
+  constexpr int kRow = N2 * N;  // pixels between a thread's elements of a column
+  const int last = sa.nslice - 1;
+  // Row-mapped: natural row ny; element i is the natural column xof(i) + rt.
+  const int ny = (r * H + ln.y + N / 2) % N, rpix = ny * N + ln.rt;
+  auto xof = [](int i) { return N2 * ((i + E / 2) % E); };
+  const size_t opix = (size_t)(corner.x + ny) * a.nxo + corner.y + ln.rt;
+  // Column-mapped: element i is the pixel (ky, kx) = (N2·i + t, r·H + c).
+  const int dpix = ln.t * N + r * H + ln.c;
 
+  // Times slice s's window (the last slice also q), or its conjugate.
+  auto window = [&](float2 (&v)[E], int s, bool conj) {
+    const float2* o = a.object + (size_t)s * sa.obj_plane + opix;
+    float2 w[E];
+#pragma unroll
+    for (int i = 0; i < E; ++i) w[i] = o[xof(i)];
+    if (s == last) {
+#pragma unroll
+      for (int i = 0; i < E; ++i) w[i] = cmul(w[i], a.quad[rpix + xof(i)]);
+    }
+#pragma unroll
+    for (int i = 0; i < E; ++i) v[i] = conj ? cmulc(w[i], v[i]) : cmul(v[i], w[i]);
+  };
+  auto rows_out = [&](const float2 (&v)[E], float2* dst) {
+#pragma unroll
+    for (int i = 0; i < E; ++i) dst[xof(i)] = v[i];
+  };
+  // The published row spectra through gap s's transfer function (or its conjugate) / N².
+  auto through_columns = [&](float2 (&v)[E], int s, bool adjoint) {
+    const float2* tf = sa.tf + (size_t)s * plane + dpix;
+#pragma unroll 1
+    for (int m = 0; m < K; ++m) {
+      ln.columns_forward(v, m);
+#pragma unroll
+      for (int i = 0; i < E; ++i) {
+        const float2 t = cscale(tf[i * kRow], inv_n2);
+        v[i] = adjoint ? cmulc(t, v[i]) : cmul(v[i], t);
+      }
+      ln.columns_inverse(v, m);
+    }
+  };
+
+  float2 v[E];
   if (MODE != kSliceBackward) {
     // Slice 0's exit wave: probe (natural) times the window, in the shifted layout.
-#pragma unroll 2
-    for (int idx = tid; idx < H * N; idx += T) {
-      const int yl = idx / N, jx = idx % N;
-      const int ny = (r * H + yl + N / 2) % N, nx = (jx + N / 2) % N;
+#pragma unroll 1
+    for (int m = 0; m < K; ++m) {
+      const float2* p = a.probe + (size_t)slot * a.probe_stride + m * plane + rpix;
+#pragma unroll
+      for (int i = 0; i < E; ++i) v[i] = p[xof(i)];
+      window(v, 0, false);
+      if (m == 0) __syncthreads();  // the twiddle table
+      ln.rows_forward(v, m);
+    }
+    L::publish();
+#pragma unroll 1
+    for (int s = 0; s < last; ++s) {
+      through_columns(v, s, false);
+      L::publish();
+#pragma unroll 1
       for (int m = 0; m < K; ++m) {
-        const int line = m * H + yl;
-        S[line * L + (jx ^ swz(line))] =
-            a.probe[(size_t)slot * a.probe_stride + ((size_t)m * N + ny) * N + nx];
+        ln.rows_inverse(v, m);
+        if (MODE == kSliceForward || MODE == kSliceGrad)
+          rows_out(v, sa.incident + s * slice_stride + slot * frame_planes + m * plane + rpix);
+        window(v, s + 1, false);
+        ln.rows_forward(v, m);
       }
+      L::publish();
     }
-    __syncthreads();
-    apply_window<N, C>(S, sa, 0, corner, r, K, false);
-    for (int s = 0; s + 1 < sa.nslice; ++s) {
-      through_gap<N, C>(S, sa.tf + (size_t)s * N * N, K, false, ltw, cluster, r);
-      if (MODE == kSliceForward || MODE == kSliceGrad)
-        rows_io<N, C>(S, sa.incident + s * slice_stride + slot * frame_planes, r, K, true);
-      apply_window<N, C>(S, sa, s + 1, corner, r, K, false);
-    }
-    all_lines<N, C, -1>(S, K * H, ltw);
-    transpose<N, C>(S, K, cluster);
-    all_lines<N, C, -1>(S, K * H, ltw);
-  } else {
-    const float2* src = a.field + ((size_t)slot * C + r) * K * H * N;
-#pragma unroll 8
-    for (int idx = tid; idx < K * H * N; idx += T) {
-      const int line = idx / N, e = idx % N;
-      S[line * L + (e ^ swz(line))] = src[idx];
-    }
-    __syncthreads();
   }
 
-  // Detector plane (column strips): xi pass, LLK, projection, as the frame kernel.
-  constexpr int kPix = H * N / T;
-  const float* iobs = a.iobs + (size_t)f * N * N;
-  float yo_r[kPix], ic_r[kPix];
+  // Detector plane: xi pass, LLK, projection, as the frame kernel.
+  float yo[E], ic[E];
+  {
+    const float* iobs = a.iobs + (size_t)f * plane + dpix;
 #pragma unroll
-  for (int i = 0; i < kPix; ++i) {
-    const int idx = tid + i * T;
-    const int c = idx % H, ky = idx / H;
-    yo_r[i] = iobs[ky * N + r * H + c];
-    float ic = 0.f;
-    for (int m = 0; m < K; ++m) ic += cnorm2(S[(m * H + c) * L + (ky ^ swz(m * H + c))]);
-    ic_r[i] = ic * inv_n2;
+    for (int i = 0; i < E; ++i) {
+      yo[i] = iobs[i * kRow];
+      ic[i] = 0.f;
+    }
   }
+  float2* field = a.field + ((size_t)slot * C + r) * K * H * N + tid;
+#pragma unroll 1
+  for (int m = 0; m < K; ++m) {
+    if (MODE == kSliceBackward) {
+#pragma unroll
+      for (int i = 0; i < E; ++i) v[i] = field[(size_t)m * H * N + i * T];
+    } else {
+      ln.columns_forward(v, m);
+    }
+    if (MODE == kSliceForward) {
+#pragma unroll
+      for (int i = 0; i < E; ++i) field[(size_t)m * H * N + i * T] = v[i];
+    }
+#pragma unroll
+    for (int i = 0; i < E; ++i) ic[i] += cnorm2(v[i]);
+    // the last mode stays in registers
+    if ((MODE == kSliceBackward || MODE == kSliceGrad) && m + 1 < K) ln.stash(v, m);
+  }
+  if (MODE == kSliceBackward) __syncthreads();  // the twiddle table
+#pragma unroll
+  for (int i = 0; i < E; ++i) ic[i] *= inv_n2;
   if (MODE == kSliceLlk) {
     double acc[4] = {0.0, 0.0, 0.0, 0.0};
 #pragma unroll
-    for (int i = 0; i < kPix; ++i) {
-      const float yo = yo_r[i], ic = ic_r[i];
-      if (yo < 0.f) continue;
-      acc[0] += yo > 0.f ? (double)ic - yo + (double)yo * log((double)yo / ic) : (double)ic;
-      const double dg = (double)yo - ic;
-      acc[1] += dg * dg / ((double)yo + 1.0);
-      const double de = sqrt((double)yo) - sqrt((double)ic);
+    for (int i = 0; i < E; ++i) {
+      if (yo[i] < 0.f) continue;
+      const double y = yo[i], c = ic[i];
+      acc[0] += yo[i] > 0.f ? c - y + y * log(y / c) : c;
+      const double dg = y - c;
+      acc[1] += dg * dg / (y + 1.0);
+      const double de = sqrt(y) - sqrt(c);
       acc[2] += 4.0 * de * de;
-      acc[3] += ic;
+      acc[3] += c;
     }
     block_sum<T>(acc, 4, red);
     csync<C>(cluster);
@@ -203,10 +213,9 @@ __global__ void __launch_bounds__(FrameShape<N, C>::T, frame_min_blocks<N, C>())
                             : batch_mean(a.a_mid, a.frames, 0, a.nslot, red + 7);
     double num = 0.0, den = 0.0;
 #pragma unroll
-    for (int i = 0; i < kPix; ++i) {
-      const float yo = yo_r[i];
-      if (yo < 0.f) continue;
-      const double yp = (double)ic_r[i], yt = yo;
+    for (int i = 0; i < E; ++i) {
+      if (yo[i] < 0.f) continue;
+      const double yp = (double)ic[i], yt = yo[i];
       const double xi = 1.0 - yt / (yp + 1e-5);
       num += xi * (yp - yt / (1.0 - prev * xi));
       den += xi * xi * yp;
@@ -218,67 +227,60 @@ __global__ void __launch_bounds__(FrameShape<N, C>::T, frame_min_blocks<N, C>())
   } else if (MODE == kSliceBackward && r == 0 && tid == 0) {
     a.a_out[slot] = afar;
   }
-  if (MODE == kSliceForward) {
-    float2* dst = a.field + ((size_t)slot * C + r) * K * H * N;
-#pragma unroll 8
-    for (int idx = tid; idx < K * H * N; idx += T) {
-      const int line = idx / N, e = idx % N;
-      dst[idx] = S[line * L + (e ^ swz(line))];
-    }
-    return;
-  }
+  if (MODE == kSliceForward) return;
 #pragma unroll
-  for (int i = 0; i < kPix; ++i) {
-    const int idx = tid + i * T;
-    const int c = idx % H, ky = idx / H;
-    const float yo = yo_r[i], ic = ic_r[i];
+  for (int i = 0; i < E; ++i) {
+    const float y = yo[i], c = ic[i];
     float fac;
     if (MODE == kSliceGrad) {
       // GradPoissonFourier (engine/ops.rs:161-195), or BH's (engine/bh.rs:168-275)
-      fac = yo < 0.f                ? 0.f
-            : a.cost == kCostBh     ? 2.f * (1.f - sqrtf(yo) / (sqrtf(ic) + 1e-8f))
-                                    : 2.f * (1.f - yo / fmaxf(ic, 1e-12f));
+      fac = y < 0.f             ? 0.f
+            : a.cost == kCostBh ? 2.f * (1.f - sqrtf(y) / (sqrtf(c) + 1e-8f))
+                                : 2.f * (1.f - y / fmaxf(c, 1e-12f));
       fac *= inv_n2;
     } else {
       float cres = 0.f;
-      if (yo >= 0.f)
-        cres = a.cost == kCostPoisson ? 1.f - yo / (ic + 1e-6f)
-                                      : 2.f * (1.f - sqrtf(fmaxf(yo, 0.f)) / (sqrtf(ic) + 1e-9f));
+      if (y >= 0.f)
+        cres = a.cost == kCostPoisson ? 1.f - y / (c + 1e-6f)
+                                      : 2.f * (1.f - sqrtf(fmaxf(y, 0.f)) / (sqrtf(c) + 1e-9f));
       fac = (1.f - afar * cres) * inv_n2;
     }
-    for (int m = 0; m < K; ++m) {
-      float2& v = S[(m * H + c) * L + (ky ^ swz(m * H + c))];
-      v = cscale(v, fac);
-    }
+    ic[i] = fac;
   }
-  __syncthreads();
-  all_lines<N, C, +1>(S, K * H, ltw);
-  transpose<N, C>(S, K, cluster);
-  all_lines<N, C, +1>(S, K * H, ltw);
-  // χ of the last slice: ψ' − q·O_last·in_last (the gradient: ψ' itself).
-  const int last = sa.nslice - 1;
-  const float2* in_last = last == 0 ? nullptr : sa.incident + (last - 1) * slice_stride + slot * frame_planes;
-  const float2* obj_last = a.object + (size_t)last * sa.obj_plane;
-#pragma unroll 2
-  for (int idx = tid; idx < (MODE == kSliceGrad ? 0 : H * N); idx += T) {
-    const int yl = idx / N, jx = idx % N;
-    const int ny = (r * H + yl + N / 2) % N, nx = (jx + N / 2) % N;
-    const float2 oq =
-        cmul(obj_last[(size_t)(corner.x + ny) * a.nxo + corner.y + nx], a.quad[ny * N + nx]);
-    for (int m = 0; m < K; ++m) {
-      const int line = m * H + yl;
-      const size_t pi = ((size_t)m * N + ny) * N + nx;
-      const float2 in = in_last ? in_last[pi] : a.probe[(size_t)slot * a.probe_stride + pi];
-      float2& v = S[line * L + (jx ^ swz(line))];
-      v = csub(v, cmul(in, oq));
-    }
+#pragma unroll 1
+  for (int m = K - 1; m >= 0; --m) {
+    if (m + 1 < K) ln.unstash(v, m);
+#pragma unroll
+    for (int i = 0; i < E; ++i) v[i] = cscale_rn(v[i], ic[i]);
+    ln.columns_inverse(v, m);
   }
-  __syncthreads();
-  rows_io<N, C>(S, sa.chi + last * slice_stride + slot * frame_planes, r, K, true);
-  for (int s = last - 1; s >= 0; --s) {
-    apply_window<N, C>(S, sa, s + 1, corner, r, K, true);
-    through_gap<N, C>(S, sa.tf + (size_t)s * N * N, K, true, ltw, cluster, r);
-    rows_io<N, C>(S, sa.chi + s * slice_stride + slot * frame_planes, r, K, true);
+  L::publish();
+  // χ of the last slice: ψ' − q·O_last·in_last (the gradient: ψ' itself), then slice by slice
+  // back through conj(q·O) and the gap's adjoint.
+#pragma unroll 1
+  for (int s = last;; --s) {
+#pragma unroll 1
+    for (int m = 0; m < K; ++m) {
+      const size_t pi = slot * frame_planes + m * plane + rpix;
+      ln.rows_inverse(v, m);
+      if (MODE == kSliceBackward && s == last) {
+        const float2* in = last == 0 ? a.probe + (size_t)slot * a.probe_stride + m * plane + rpix
+                                     : sa.incident + (last - 1) * slice_stride + pi;
+        const float2* o = a.object + (size_t)last * sa.obj_plane + opix;
+#pragma unroll
+        for (int i = 0; i < E; ++i)
+          v[i] = csub(v[i], cmul(in[xof(i)], cmul(o[xof(i)], a.quad[rpix + xof(i)])));
+      }
+      rows_out(v, sa.chi + s * slice_stride + pi);
+      if (s > 0) {
+        window(v, s, true);
+        ln.rows_forward(v, m);
+      }
+    }
+    if (s == 0) break;
+    L::publish();
+    through_columns(v, s - 1, true);
+    L::publish();
   }
 }
 

@@ -86,15 +86,16 @@ cudaError_t move_modes(int mode, const MoveArgs& a, int nslot, int K, cudaStream
 
 template <int N, int C>
 cudaError_t slice_modes(int mode, const SliceArgs& a, int nslot, int K, cudaStream_t s) {
+  constexpr int T = PlaneShape<N, C>::T;
   const size_t smem = frame_smem_bytes<N, C>(K);
   switch (mode) {
     case kSliceForward:
-      return launch_clusters<N, C>(slice_kernel<N, C, kSliceForward>, a, nslot, smem, s);
+      return launch_clusters<N, C, T>(slice_kernel<N, C, kSliceForward>, a, nslot, smem, s);
     case kSliceBackward:
-      return launch_clusters<N, C>(slice_kernel<N, C, kSliceBackward>, a, nslot, smem, s);
-    case kSliceLlk: return launch_clusters<N, C>(slice_kernel<N, C, kSliceLlk>, a, nslot, smem, s);
+      return launch_clusters<N, C, T>(slice_kernel<N, C, kSliceBackward>, a, nslot, smem, s);
+    case kSliceLlk: return launch_clusters<N, C, T>(slice_kernel<N, C, kSliceLlk>, a, nslot, smem, s);
     case kSliceGrad:
-      return launch_clusters<N, C>(slice_kernel<N, C, kSliceGrad>, a, nslot, smem, s);
+      return launch_clusters<N, C, T>(slice_kernel<N, C, kSliceGrad>, a, nslot, smem, s);
   }
   return cudaErrorInvalidValue;
 }
