@@ -25,7 +25,24 @@ PTYB_D float2 cmulc_rn(float2 a, float2 b) {
   return make_float2(fmaf(a.x, b.x, a.y * b.y), fmaf(a.x, b.y, -(a.y * b.x)));
 }
 PTYB_HD float2 cscale(float2 a, float s) { return make_float2(a.x * s, a.y * s); }
-// The same, not contracted into an addition that follows.
+// a + b and a − b as one packed instruction each (both components per issue slot).
+PTYB_D float2 cadd2(float2 a, float2 b) {
+  float2 r;
+  asm("{.reg .b64 x, y, z; mov.b64 x, {%2, %3}; mov.b64 y, {%4, %5}; add.rn.f32x2 z, x, y; "
+      "mov.b64 {%0, %1}, z;}"
+      : "=f"(r.x), "=f"(r.y)
+      : "f"(a.x), "f"(a.y), "f"(b.x), "f"(b.y));
+  return r;
+}
+PTYB_D float2 csub2(float2 a, float2 b) {
+  float2 r;
+  asm("{.reg .b64 x, y, z, m; mov.b64 x, {%2, %3}; mov.b64 y, {%4, %5}; mov.b64 m, {%6, %6}; "
+      "fma.rn.f32x2 z, y, m, x; mov.b64 {%0, %1}, z;}"
+      : "=f"(r.x), "=f"(r.y)
+      : "f"(a.x), "f"(a.y), "f"(b.x), "f"(b.y), "f"(-1.f));
+  return r;
+}
+// cscale, not contracted into an addition that follows.
 PTYB_D float2 cscale_rn(float2 a, float s) {
   return make_float2(__fmul_rn(a.x, s), __fmul_rn(a.y, s));
 }
