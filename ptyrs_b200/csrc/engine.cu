@@ -243,22 +243,23 @@ void end_call(ptyb_handle* h, const char* what) {
 }
 
 // Cluster size for frames of side N with K modes: `want` if it is built and fits shared
-// memory, else the smallest that fits with at least two CTAs per SM, else the smallest that
-// fits; 0 when none does.
+// memory, else the largest built, which has the smallest CTAs (256 threads at sides 128 and 256):
+// more of them interleave on an SM. Clusters of 4 against 2 at 128² and 16 against 8 at 256² were
+// ahead in every algorithm at one mode too: AP 128² 5201 -> 5069 us a call of 1250 frames, rPIE
+// with positions 858 -> 807 (300 frames), DM 256² 9904 -> 9261 (1024), ML with positions 32.5 ->
+// 31.1 ms (2000), and by 1 to 5 % over 64 frames. 0 when none fits.
 int cluster_for(int N, int K, int want) {
-  const size_t lim = 227 * 1024, two = 113 * 1024;
+  const size_t lim = 227 * 1024;
   struct Opt {
     int n, c;
     size_t bytes;
   };
-  const Opt opts[] = {{64, 1, frame_smem_bytes<64, 1>(K)},   {96, 2, frame_smem_bytes<96, 2>(K)},
-                      {128, 2, frame_smem_bytes<128, 2>(K)}, {128, 4, frame_smem_bytes<128, 4>(K)},
-                      {192, 8, frame_smem_bytes<192, 8>(K)}, {256, 8, frame_smem_bytes<256, 8>(K)},
-                      {256, 16, frame_smem_bytes<256, 16>(K)}};
+  const Opt opts[] = {{64, 1, move_smem_bytes<64, 1>(K)},    {96, 2, move_smem_bytes<96, 2>(K)},
+                      {128, 4, move_smem_bytes<128, 4>(K)},  {128, 2, move_smem_bytes<128, 2>(K)},
+                      {192, 8, move_smem_bytes<192, 8>(K)},  {256, 16, move_smem_bytes<256, 16>(K)},
+                      {256, 8, move_smem_bytes<256, 8>(K)}};
   for (const Opt& o : opts)
     if (o.n == N && o.c == want && o.bytes <= lim) return o.c;
-  for (const Opt& o : opts)
-    if (o.n == N && o.bytes <= two) return o.c;
   for (const Opt& o : opts)
     if (o.n == N && o.bytes <= lim) return o.c;
   return 0;
@@ -880,7 +881,7 @@ int create_handle(const ptyb_scan* scan, const double* object, int32_t nobj, int
   // The position sums reduce over the whole cluster once per frame: at side 256 they run on
   // clusters of 8 (measured faster than 16), whatever cluster the frame kernels take.
   h->C_sums = C;
-  if (N == 256 && frame_smem_bytes<256, 8>(std::max(K, 2)) <= 227 * 1024) h->C_sums = 8;
+  if (N == 256 && move_smem_bytes<256, 8>(std::max(K, 2)) <= 227 * 1024) h->C_sums = 8;
   h->stack = options && options->stack_size > 0 ? options->stack_size : 512;
   h->nslice = nslice;
   h->log_stride = 2 + nslice;

@@ -258,7 +258,9 @@ PTYB_D void carry_mix(const FrameArgs& a, float2 (&v)[PlaneShape<N, C>::E], size
 }
 
 template <int N, int C, int MODE>
-__global__ void __launch_bounds__(PlaneShape<N, C>::T, plane_min_blocks<N, C>())
+__global__ void __launch_bounds__(PlaneShape<N, C>::T,
+                                  plane_min_blocks<N, C>(MODE == kMlGrad || MODE == kBhGrad ||
+                                                         MODE == kProjectKept))
     frame_kernel(FrameArgs a) {
   using L = Lines<N, C>;
   constexpr int H = L::H, T = L::T, E = L::N1, N2 = L::N2;

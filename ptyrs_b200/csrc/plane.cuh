@@ -34,10 +34,16 @@ struct PlaneShape {
 };
 
 // CTAs per SM the plane kernels are compiled for: 512 threads (128 registers each) where a
-// thread holds 16 elements, 1024 at side 64 (8 elements), two CTAs of 192 at 24 elements.
+// thread holds 16 elements, 1024 at side 64 (8 elements), two CTAs of 192 at 24 elements. A
+// kernel that holds little beside its line (`light`) takes 768 threads of 80 registers at side
+// 256: moves 0.906 -> 0.797 us per frame of 256² x 2, their spectra 0.998 -> 0.896, projection
+// 1.211 -> 1.055, gradient 1.941 -> 1.871, where the line search (2.46 -> 3.25), the carry pass
+// (2.21 -> 2.69) and at side 128 the LSQML passes (0.618 -> 0.757) spill and lose.
 template <int N, int C>
-__host__ __device__ constexpr int plane_min_blocks() {
-  return N == 64 ? 2 : LineShape<N>::N1 == 24 ? 2 : 512 / PlaneShape<N, C>::T;
+__host__ __device__ constexpr int plane_min_blocks(bool light = false) {
+  return N == 64 ? 2
+         : LineShape<N>::N1 == 24 ? 2
+         : (light && N == 256 && PlaneShape<N, C>::T == 256 ? 768 : 512) / PlaneShape<N, C>::T;
 }
 
 PTYB_D float2 lds2(unsigned a) {

@@ -61,7 +61,9 @@ __host__ __device__ constexpr size_t move_smem_bytes(int K) {
 // 256² x 2 modes: moves from the spectrum 1.42 -> 0.93 us, probe gradient spectra 1.57 -> 1.03,
 // position sums 3.21 -> 2.21 (four inverse transforms), one plane's spectrum 27 -> 16 us a call.
 template <int N, int C, int MODE>
-__global__ void __launch_bounds__(PlaneShape<N, C>::T, plane_min_blocks<N, C>())
+__global__ void __launch_bounds__(PlaneShape<N, C>::T,
+                                  plane_min_blocks<N, C>(MODE != kDerivSums &&
+                                                         MODE != kDerivWindow))
     move_kernel(MoveArgs a) {
   using L = Lines<N, C>;
   constexpr int H = L::H, T = L::T, E = L::N1, N2 = L::N2;
