@@ -85,3 +85,18 @@ PTYB_D float warp_max(float v) {
   for (int o = 16; o > 0; o >>= 1) v = fmaxf(v, __shfl_xor_sync(0xffffffffu, v, o));
   return v;
 }
+
+// v[i0] + v[i0+1] + … + v[i1−1] in that order by one thread, eight loads ahead of the additions.
+PTYB_D double ordered_sum(const double* v, int i0, int i1) {
+  double s = 0.0;
+  int i = i0;
+  for (; i + 8 <= i1; i += 8) {
+    double a[8];
+#pragma unroll
+    for (int k = 0; k < 8; ++k) a[k] = v[i + k];
+#pragma unroll
+    for (int k = 0; k < 8; ++k) s += a[k];
+  }
+  for (; i < i1; ++i) s += v[i];
+  return s;
+}

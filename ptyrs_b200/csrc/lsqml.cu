@@ -16,6 +16,16 @@ __global__ void fill_kernel(float* x, float v, int n) {
   if (i < n) x[i] = v;
 }
 
+// `obj` += scal[2 + which]·d_obj over `no` values and, with `np`, the probe += scal[3]·d_probe.
+void step_arrays(ptyb_handle* h, float2* obj, const float2* d_obj, int which, size_t no,
+                 size_t np) {
+  timed(h, kKAxpy, [&] {
+    axpy_scal_kernel<<<(unsigned)((no + 511) / 512 + (np + 511) / 512), 256, 0, h->stream>>>(
+        obj, d_obj, which, no, h->probe, h->d_probe, 1, np, h->scal + 2);
+  });
+  launched(h, "step");
+}
+
 // The preconditioner over every view on pty-chi's schedule (engine/lsqml.rs:676-700).
 void lsqml_preconditioner(ptyb_handle* h, bool init) {
   GatherArgs g = gather_args(h, h->iota, h->P);
@@ -174,22 +184,14 @@ void lsqml_batch_slices(ptyb_handle* h, const ptyb_lsqml_params& p, const int* f
   });
   launched(h, "step solve");
   for (int s = 0; s < S; ++s) {
-    const int which = s == 0 ? 0 : 1 + s;  // relative to scal + 2: so_0, sp, so_1, so_2, …
-    timed(h, kKAxpy, [&] {
-      axpy_scal_kernel<<<(unsigned)((no + 255) / 256), 256, 0, h->stream>>>(
-          h->object + s * no, h->d_obj + s * no, h->scal + 2, which, no);
-    });
-    launched(h, "slice step");
+    // relative to scal + 2: so_0, sp, so_1, so_2, …; the probe's step goes with slice 0's
+    const int which = s == 0 ? 0 : 1 + s;
+    step_arrays(h, h->object + s * no, h->d_obj + s * no, which, no, s == 0 ? fplanes : 0);
   }
-  timed(h, kKAxpy, [&] {
-    axpy_scal_kernel<<<(unsigned)((fplanes + 255) / 256), 256, 0, h->stream>>>(
-        h->probe, h->d_probe, h->scal + 2, 1, fplanes);
-  });
-  launched(h, "probe step");
   if (refine) {
     const double eps = 1e-6 * ((double)h->N * h->N);
     timed(h, kKSolve, [&] {
-      position_step_kernel<<<1, 32, 0, h->stream>>>(h->pos_sums, nslot, h->P, eps, frames,
+      position_step_kernel<<<1, 1024, 0, h->stream>>>(h->pos_sums, nslot, h->P, eps, frames,
                                                     h->offsets);
     });
     launched(h, "position step");
@@ -334,10 +336,7 @@ void lsqml_batch(ptyb_handle* h, const ptyb_lsqml_params& p, const int* frames, 
     check(h, launch_frame<kFromStore>(h, a, nslot), "lsqml backward");
     ++h->launches;
   } else {
-    timed(h, kKMisc, [&] {
-      fill_kernel<<<(nslot + 255) / 256, 256, 0, h->stream>>>(h->afar2, 0.5f, nslot);
-    });
-    launched(h, "a_far");
+    // h->afar2 holds the amplitude cost's constant step for the whole call (ptyb_lsqml)
     check(h, launch_frame<kLsqmlFused>(h, a, nslot), "lsqml pass");
     ++h->launches;
   }
@@ -383,20 +382,11 @@ void lsqml_batch(ptyb_handle* h, const ptyb_lsqml_params& p, const int* frames, 
   });
   launched(h, "step solve");
   const size_t no = (size_t)h->nyo * h->nxo, np = (size_t)h->K * h->N * h->N;
-  timed(h, kKAxpy, [&] {
-    axpy_scal_kernel<<<(unsigned)((no + 255) / 256), 256, 0, h->stream>>>(h->object, h->d_obj,
-                                                                         h->scal + 2, 0, no);
-  });
-  launched(h, "object step");
-  timed(h, kKAxpy, [&] {
-    axpy_scal_kernel<<<(unsigned)((np + 255) / 256), 256, 0, h->stream>>>(h->probe, h->d_probe,
-                                                                         h->scal + 2, 1, np);
-  });
-  launched(h, "probe step");
+  step_arrays(h, h->object, h->d_obj, 0, no, np);
   if (refine) {
     const double eps = 1e-6 * ((double)h->N * h->N);
     timed(h, kKSolve, [&] {
-      position_step_kernel<<<1, 32, 0, h->stream>>>(h->pos_sums, nslot, h->P, eps, frames,
+      position_step_kernel<<<1, 1024, 0, h->stream>>>(h->pos_sums, nslot, h->P, eps, frames,
                                                     h->offsets);
     });
     launched(h, "position step");
@@ -440,6 +430,12 @@ int ptyb_lsqml(ptyb_handle* h, const ptyb_lsqml_params* p, int32_t nepoch, int32
       fill_kernel<<<(h->P + 255) / 256, 256, 0, h->stream>>>(h->afar_all, 0.5f, h->P);
     });
     launched(h, "a_far");
+    if (p->cost == PTYB_COST_AMPLITUDE) {
+      timed(h, kKMisc, [&] {
+        fill_kernel<<<(size + 255) / 256, 256, 0, h->stream>>>(h->afar2, 0.5f, size);
+      });
+      launched(h, "a_far");
+    }
     for (int ic = 0; ic < nepoch; ++ic) {
       if (ic < 10 || ic % 10 == 0) lsqml_preconditioner(h, ic == 0);
       const int* order = h->order_all + (size_t)ic * h->P;

@@ -134,12 +134,32 @@ static __global__ void __launch_bounds__(1024) lsqml_solve_kernel(const double* 
   }
 }
 
-// x += scal[which]·d over n values.
-static __global__ void axpy_scal_kernel(float2* x, const float2* d, const float* scal, int which,
-                                 size_t n) {
-  const size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= n) return;
-  x[i] = cadd(x[i], cscale(d[i], scal[which]));
+// x += a·d over values 2i and 2i + 1, in 16-byte accesses where both arrays lie on 16-byte
+// boundaries (every second slice of an odd number of values does not).
+PTYB_D void axpy_pairs(float2* x, const float2* d, float a, size_t n, size_t i) {
+  const bool wide = ((reinterpret_cast<size_t>(x) | reinterpret_cast<size_t>(d)) & 15) == 0;
+  if (wide && 2 * i + 1 < n) {
+    float4 v = reinterpret_cast<float4*>(x)[i];
+    const float4 w = reinterpret_cast<const float4*>(d)[i];
+    const float2 p = cadd(make_float2(v.x, v.y), cscale(make_float2(w.x, w.y), a));
+    const float2 q = cadd(make_float2(v.z, v.w), cscale(make_float2(w.z, w.w), a));
+    reinterpret_cast<float4*>(x)[i] = make_float4(p.x, p.y, q.x, q.y);
+  } else {
+    for (size_t j = 2 * i; j < n && j < 2 * i + 2; ++j) x[j] = cadd(x[j], cscale(d[j], a));
+  }
+}
+
+// The batch's object and probe steps in one launch: x0 += scal[which0]·d0 over n0 values, then
+// x1 += scal[which1]·d1 over n1 (n1 0: none).
+static __global__ void __launch_bounds__(256) axpy_scal_kernel(float2* x0, const float2* d0,
+                                                               int which0, size_t n0, float2* x1,
+                                                               const float2* d1, int which1,
+                                                               size_t n1, const float* scal) {
+  const size_t b0 = (n0 + 511) / 512;
+  if (blockIdx.x < b0)
+    axpy_pairs(x0, d0, scal[which0], n0, (size_t)blockIdx.x * 256 + threadIdx.x);
+  else
+    axpy_pairs(x1, d1, scal[which1], n1, (size_t)(blockIdx.x - b0) * 256 + threadIdx.x);
 }
 
 // Max of a non-negative float array into *out (which starts at 0).

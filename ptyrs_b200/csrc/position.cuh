@@ -339,27 +339,62 @@ static __global__ void __launch_bounds__(256) position_sums_kernel(const float2*
   }
 }
 
-// pty-chi's gradient position step on the batch (engine/features.rs:496-521), one thread in
-// double: delta = num/(den + max(max_batch den, eps)), dx = 0.3·delta at the batch's frames
-// (0 elsewhere), each axis clipped to min(10·mean|dx − mean dx|, 0.1) over every frame.
-static __global__ void position_step_kernel(const double* sums, int nslot, int nframe, double eps,
-                                     const int* frames, double* offsets) {
-  if (threadIdx.x != 0 || blockIdx.x != 0) return;
-  for (int a = 0; a < 2; ++a) {
-    double mx = eps;
-    for (int s = 0; s < nslot; ++s) mx = fmax(mx, sums[s * 4 + 2 + a]);
-    double total = 0.0;
-    for (int s = 0; s < nslot; ++s) total += 0.3 * (sums[s * 4 + a] / (sums[s * 4 + 2 + a] + mx));
-    const double mean = total / nframe;
-    double dev = (double)(nframe - nslot) * fabs(mean);
-    for (int s = 0; s < nslot; ++s)
-      dev += fabs(0.3 * (sums[s * 4 + a] / (sums[s * 4 + 2 + a] + mx)) - mean);
-    const double limit = fmin(10.0 * (dev / nframe), 0.1);
-    for (int s = 0; s < nslot; ++s) {
-      const double dx = 0.3 * (sums[s * 4 + a] / (sums[s * 4 + 2 + a] + mx));
-      offsets[2 * frames[s] + a] += fmin(fmax(dx, -limit), limit);
-    }
+// pty-chi's gradient position step on the batch (engine/features.rs:496-521) in double, one
+// block: delta = num/(den + max(max_batch den, eps)), dx = 0.3·delta at the batch's frames
+// (0 elsewhere), each axis clipped to min(10·mean|dx − mean dx|, 0.1) over every frame. The
+// sums run in slot order, one warp per axis, over terms every thread forms (by one thread alone,
+// its divisions took 113 us a batch of 150).
+static __global__ void __launch_bounds__(1024) position_step_kernel(const double* sums, int nslot,
+                                                                    int nframe, double eps,
+                                                                    const int* frames,
+                                                                    double* offsets) {
+  __shared__ double term[2][1024], red[2][32], mx[2], acc[2];
+  const int t = threadIdx.x;
+  double m0 = eps, m1 = eps;
+  for (int s = t; s < nslot; s += 1024) {
+    m0 = fmax(m0, sums[s * 4 + 2]);
+    m1 = fmax(m1, sums[s * 4 + 3]);
   }
+  for (int o = 16; o > 0; o >>= 1) {
+    m0 = fmax(m0, __shfl_xor_sync(0xffffffffu, m0, o));
+    m1 = fmax(m1, __shfl_xor_sync(0xffffffffu, m1, o));
+  }
+  if (t % 32 == 0) {
+    red[0][t / 32] = m0;
+    red[1][t / 32] = m1;
+  }
+  __syncthreads();
+  if (t < 2) {
+    double m = eps;
+    for (int w = 0; w < 32; ++w) m = fmax(m, red[t][w]);
+    mx[t] = m;
+  }
+  __syncthreads();
+  auto dx = [&](int s, int a) { return 0.3 * (sums[s * 4 + a] / (sums[s * 4 + 2 + a] + mx[a])); };
+  // Σ f(dx) over the slots in order, per axis, into acc[axis]
+  auto sum = [&](auto f) {
+    if (t < 2) acc[t] = 0.0;
+    for (int s0 = 0; s0 < nslot; s0 += 1024) {
+      const int n = min(1024, nslot - s0);
+      if (t < n) {
+        term[0][t] = f(dx(s0 + t, 0), 0);
+        term[1][t] = f(dx(s0 + t, 1), 1);
+      }
+      __syncthreads();
+      if (t == 0 || t == 32) acc[t / 32] += ordered_sum(term[t / 32], 0, n);
+      __syncthreads();
+    }
+  };
+  sum([](double x, int) { return x; });
+  const double mean[2] = {acc[0] / nframe, acc[1] / nframe};
+  __syncthreads();
+  sum([&](double x, int a) { return fabs(x - mean[a]); });
+  double limit[2];
+  for (int a = 0; a < 2; ++a)
+    limit[a] = fmin(10.0 * (((double)(nframe - nslot) * fabs(mean[a]) + acc[a]) / nframe), 0.1);
+  for (int s = t; s < nslot; s += 1024)
+    for (int a = 0; a < 2; ++a)
+      offsets[2 * frames[s] + a] += fmin(fmax(dx(s, a), -limit[a]), limit[a]);
 }
 
 // Block sum of one double per thread in a fixed order (lane trees, then warps in order).

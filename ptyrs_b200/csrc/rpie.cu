@@ -94,7 +94,7 @@ void rpie_batch(ptyb_handle* h, const ptyb_rpie_params& p, const int* frames, in
   if (refine) {
     const double eps = 1e-6 * ((double)h->N * h->N);
     timed(h, kKSolve, [&] {
-      position_step_kernel<<<1, 32, 0, h->stream>>>(h->pos_sums, nslot, h->P, eps, frames,
+      position_step_kernel<<<1, 1024, 0, h->stream>>>(h->pos_sums, nslot, h->P, eps, frames,
                                                     h->offsets);
     });
     launched(h, "position step");
