@@ -101,8 +101,7 @@ void bh_grads(ptyb_handle* h, const int* frames, int n) {
     pa.K = h->K;
     pa.N = h->N;
     pa.mode = 1;
-    dim3 grid((h->N * h->N + 255) / 256, nchunk);
-    timed(h, kKProbePartial, [&] { probe_partial_kernel<<<grid, 256, 0, h->stream>>>(pa); }, m);
+    timed(h, kKProbePartial, [&] { launch_probe_partial(pa, nchunk, h->stream); }, m);
     launched(h, "bh probe gradient");
     timed(h, kKProbeFinal, [&] {
       probe_finalize_kernel<<<(unsigned)((np + 255) / 256), 256, 0, h->stream>>>(

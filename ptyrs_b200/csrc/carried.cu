@@ -96,8 +96,7 @@ int probe_blend_sums(ptyb_handle* h, int mode = 2) {
   p.K = h->K;
   p.N = h->N;
   p.mode = mode;
-  dim3 grid((plane + 255) / 256, nchunk);
-  timed(h, kKProbePartial, [&] { probe_partial_kernel<<<grid, 256, 0, h->stream>>>(p); }, h->P);
+  timed(h, kKProbePartial, [&] { launch_probe_partial(p, nchunk, h->stream); }, h->P);
   launched(h, "probe partial");
   return nchunk;
 }

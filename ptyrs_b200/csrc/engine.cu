@@ -415,8 +415,7 @@ void probe_pass(ptyb_handle* h, const int* frames, int nslot, int mode, float al
   p.K = h->K;
   p.N = h->N;
   p.mode = mode == 0 ? 0 : 1;
-  dim3 grid((h->N * h->N + 255) / 256, nchunk);
-  timed(h, kKProbePartial, [&] { probe_partial_kernel<<<grid, 256, 0, h->stream>>>(p); }, nslot);
+  timed(h, kKProbePartial, [&] { launch_probe_partial(p, nchunk, h->stream); }, nslot);
   launched(h, "probe_partial");
   const int count = h->K * h->N * h->N;
   timed(h, kKProbeFinal, [&] {

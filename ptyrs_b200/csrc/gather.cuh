@@ -248,8 +248,11 @@ struct ProbeArgs {
 
 constexpr int kMaxProbeChunk = 256;
 
-// Chunk `blockIdx.y` of slots (at most kMaxProbeChunk), 256 probe pixels per CTA:
-// Σ_slots w·upd in slot order.
+// Chunk `blockIdx.y` of slots (at most kMaxProbeChunk), 512 probe pixels per CTA of 256 threads:
+// Σ_slots w·upd in slot order for a's K modes. Two neighbouring pixels a thread, the update
+// planes and the phase read 16 bytes at a time: bound by the latency of those loads (84 % of the
+// stalls with one pixel a thread).
+template <int K>
 static __global__ void __launch_bounds__(256) probe_partial_kernel(ProbeArgs a) {
   __shared__ int2 cs[kMaxProbeChunk];
   __shared__ float om[kMaxProbeChunk];
@@ -261,35 +264,67 @@ static __global__ void __launch_bounds__(256) probe_partial_kernel(ProbeArgs a) 
     om[i] = a.mode == 0 ? a.omax[s0 + i] : 0.f;
   }
   __syncthreads();
-  const int pix = blockIdx.x * 256 + threadIdx.x;
+  const int pix = 2 * (blockIdx.x * 256 + threadIdx.x);
   if (pix >= N * N) return;
   const int yy = pix / N, xx = pix % N;
-  const float2 q = a.quad[pix];
-  KahanC acc[kMaxModes];
-  Kahan den;
-  den.init();
+  const float4 qv = reinterpret_cast<const float4*>(a.quad)[pix / 2];
+  const float2 q[2] = {make_float2(qv.x, qv.y), make_float2(qv.z, qv.w)};
+  KahanC acc[2][K];
+  Kahan den[2];
 #pragma unroll
-  for (int m = 0; m < kMaxModes; ++m) acc[m].init();
+  for (int j = 0; j < 2; ++j) {
+    den[j].init();
+#pragma unroll
+    for (int m = 0; m < K; ++m) acc[j][m].init();
+  }
+  const float2* obj = a.object + (size_t)yy * a.nxo + xx;
 #pragma unroll 4
   for (int s = s0; s < s1; ++s) {
     const int2 c = cs[s - s0];
-    const float2 o = a.object[(size_t)(c.x + yy) * a.nxo + c.y + xx];
-    if (a.mode >= 2) den.add(cnorm2(o));
+    const float2* op = obj + (size_t)c.x * a.nxo + c.y;
+    float2 o[2] = {op[0], op[1]};
+    if (a.mode >= 2) {
+      den[0].add(cnorm2(o[0]));
+      den[1].add(cnorm2(o[1]));
+    }
     if (a.mode == 3) continue;
-    float2 w = cconj(cmul(o, q));
-    if (a.mode == 0) w = cscale(w, 1.f / ((1.f - a.alpha) * cnorm2(o) + a.alpha * om[s - s0]));
+    float2 w[2];  // conjugated in the products below
 #pragma unroll
-    for (int m = 0; m < kMaxModes; ++m) {
-      if (m >= a.K) break;
-      acc[m].add(cmul(w, a.upd[((size_t)s * a.K + m) * plane + pix]));
+    for (int j = 0; j < 2; ++j) {
+      w[j] = cmul_rn(o[j], q[j]);
+      if (a.mode == 0)
+        w[j] = cscale(w[j], 1.f / ((1.f - a.alpha) * cnorm2(o[j]) + a.alpha * om[s - s0]));
+    }
+#pragma unroll
+    for (int m = 0; m < K; ++m) {
+      const float4 u =
+          reinterpret_cast<const float4*>(a.upd + ((size_t)s * K + m) * plane)[pix / 2];
+      acc[0][m].add(cmulc_rn2(w[0], make_float2(u.x, u.y)));
+      acc[1][m].add(cmulc_rn2(w[1], make_float2(u.z, u.w)));
     }
   }
   if (a.mode != 3) {
 #pragma unroll
-    for (int m = 0; m < kMaxModes; ++m)
-      if (m < a.K) a.partial[((size_t)blockIdx.y * a.K + m) * plane + pix] = acc[m].value();
+    for (int m = 0; m < K; ++m) {
+      const float2 v0 = acc[0][m].value(), v1 = acc[1][m].value();
+      reinterpret_cast<float4*>(a.partial + ((size_t)blockIdx.y * K + m) * plane)[pix / 2] =
+          make_float4(v0.x, v0.y, v1.x, v1.y);
+    }
   }
-  if (a.mode >= 2) a.partial_den[(size_t)blockIdx.y * plane + pix] = den.s - den.c;
+  if (a.mode >= 2)
+    reinterpret_cast<float2*>(a.partial_den + (size_t)blockIdx.y * plane)[pix / 2] =
+        make_float2(den[0].s - den[0].c, den[1].s - den[1].c);
+}
+
+// One launch over `nchunk` chunks (K ≤ 4; N² is a multiple of 512 at every side).
+static inline void launch_probe_partial(const ProbeArgs& a, int nchunk, cudaStream_t s) {
+  const dim3 grid((a.N * a.N + 511) / 512, nchunk);
+  switch (a.K) {
+    case 1: probe_partial_kernel<1><<<grid, 256, 0, s>>>(a); break;
+    case 2: probe_partial_kernel<2><<<grid, 256, 0, s>>>(a); break;
+    case 3: probe_partial_kernel<3><<<grid, 256, 0, s>>>(a); break;
+    default: probe_partial_kernel<4><<<grid, 256, 0, s>>>(a);
+  }
 }
 
 // The object blend of AP / DM / RAAR (engine/ops.rs:371-381) from the sums kGatherBlend wrote:

@@ -76,8 +76,7 @@ void slice_gradients(ptyb_handle* h, bool uo, bool up, const int* frames_in, int
       pa.K = h->K;
       pa.N = h->N;
       pa.mode = 1;
-      dim3 grid((h->N * h->N + 255) / 256, nchunk);
-      timed(h, kKProbePartial, [&] { probe_partial_kernel<<<grid, 256, 0, h->stream>>>(pa); }, n);
+      timed(h, kKProbePartial, [&] { launch_probe_partial(pa, nchunk, h->stream); }, n);
       launched(h, "probe gradient");
       const int count = (int)fplanes;
       timed(h, kKProbeFinal, [&] {
@@ -183,8 +182,7 @@ void ml_gradients(ptyb_handle* h, bool uo, bool up, bool refine, bool pos_grad =
       pa.K = h->K;
       pa.N = h->N;
       pa.mode = 1;
-      dim3 grid((h->N * h->N + 255) / 256, nchunk);
-      timed(h, kKProbePartial, [&] { probe_partial_kernel<<<grid, 256, 0, h->stream>>>(pa); }, pa.nslot);
+      timed(h, kKProbePartial, [&] { launch_probe_partial(pa, nchunk, h->stream); }, pa.nslot);
       launched(h, "probe gradient");
       const int count = h->K * h->N * h->N;
       timed(h, kKProbeFinal, [&] {

@@ -72,8 +72,7 @@ void rpie_batch(ptyb_handle* h, const ptyb_rpie_params& p, const int* frames, in
     pa.K = h->K;
     pa.N = h->N;
     pa.mode = 0;
-    dim3 grid((h->N * h->N + 255) / 256, nchunk);
-    timed(h, kKProbePartial, [&] { probe_partial_kernel<<<grid, 256, 0, h->stream>>>(pa); }, pa.nslot);
+    timed(h, kKProbePartial, [&] { launch_probe_partial(pa, nchunk, h->stream); }, pa.nslot);
     launched(h, "probe partial");
   }
   if (p.update_object) {
