@@ -332,7 +332,6 @@ FrameArgs frame_args(ptyb_handle* h, const int* frames) {
 
 GatherArgs gather_args(ptyb_handle* h, const int* frames, int nslot) {
   GatherArgs g = {};
-  g.object = h->object;
   g.probe = h->probe;
   g.quad = h->quad;
   g.upd = h->upd;

@@ -161,6 +161,11 @@ struct ptyb_handle {
   double* pcg_norms = nullptr;    // [P][K]
   double* pcg_modes = nullptr;    // [K][2]
   double* partials = nullptr;    // [kPartialBlocks][2]
+  // rPIE: a batch's object sums and overlaps per mode [K][nyo][nxo], the largest overlap of this
+  // batch and the next.
+  float2* rpie_num = nullptr;
+  float* rpie_den = nullptr;
+  float* rpie_max = nullptr;
   // Phase-ramp removal: the probe's row transforms [K][N][N], the columns' sums [K·N][3] and
   // the centroid's offset (dy, dx) behind them.
   double2* ramp_rows = nullptr;

@@ -18,27 +18,26 @@ constexpr int kGroups = 4;     // view groups per pixel
 constexpr int kMaxModes = 4;
 
 enum GatherMode : int {
-  kGatherRpie = 0,   // O += step·Σ_m num_m / ((1−α)·D_m + α·pmax)
+  kGatherRpie = 0,   // rPIE's sums: out = num_m, pre = D_m (−1 where no view covers the pixel),
+                     // pmax = max over pixels of Σ_m D_m
   kGatherLsqml = 1,  // d_obj = Σ conj(q·P)·χ / √(pre² + floor²)
   kGatherMl = 2,     // grad += Σ conj(q·P)·g (compensated across launches)
-  kGatherOverlap = 3,  // pmax = max over pixels of Σ_m D_m
   kGatherIllum = 4,    // pre = (pre + I)/2 with I = Σ|P|² over every view
   kGatherBlend = 5,    // the object blend's sums: out = num, pre = norm, pmax = max norm
 };
 
 struct GatherArgs {
-  float2* object;          // [nyo][nxo] object mode 0 (rPIE updates it)
   const float2* probe;     // [nprobe][N][N]
   const float2* quad;      // [N][N]
   const float2* upd;       // [slot][K][N][N] natural: Δ, χ or g
   const int* frames;       // [nslot]
   const int2* corners;     // [nframe]
   float* pmax;             // rPIE overlap max (device scalar)
-  float* pre;              // LSQML preconditioner [nyo][nxo]
+  float* pre;              // LSQML preconditioner [nyo][nxo], rPIE [K][nyo][nxo]
   const float* pre_max;    // LSQML: max of pre (device scalar)
-  float2* out;             // LSQML d_obj / ML gradient sum [nyo][nxo]
+  float2* out;             // LSQML d_obj / ML gradient sum [nyo][nxo], rPIE [K][nyo][nxo]
   float2* comp;            // ML gradient compensation [nyo][nxo]
-  float alpha, step, pre_scale;
+  float pre_scale;
   int nslot, nyo, nxo, nprobe, N;
   int probe_stride;        // elements between slots' probes (0: the shared probe)
 };
@@ -85,7 +84,7 @@ PTYB_D int tile_list(const GatherArgs& a, int s0, int s1, int ty0, int tx0, int*
 }
 
 template <int MODE>
-__global__ void __launch_bounds__(1024, MODE == kGatherRpie || MODE == kGatherBlend ? 1 : 2) object_tile_kernel(GatherArgs a) {
+PTYB_D void object_tile(const GatherArgs& a) {
   constexpr int kChunk = 1024;
   constexpr int kPix = kTile * kTile;  // 256 pixels, kGroups threads each
   // The view list (during the walk), then the groups' partial sums (after it).
@@ -139,8 +138,7 @@ __global__ void __launch_bounds__(1024, MODE == kGatherRpie || MODE == kGatherBl
       for (int m = 0; m < kMaxModes; ++m) {
         if (m >= K) break;
         const float2 p = a.probe[(size_t)s * a.probe_stride + m * plane + pix];
-        if (MODE == kGatherOverlap || MODE == kGatherIllum || MODE == kGatherRpie ||
-            MODE == kGatherBlend)
+        if (MODE == kGatherIllum || MODE == kGatherRpie || MODE == kGatherBlend)
           den[m].add(cnorm2(p));
         if (MODE == kGatherRpie || MODE == kGatherLsqml || MODE == kGatherMl ||
             MODE == kGatherBlend) {
@@ -176,7 +174,7 @@ __global__ void __launch_bounds__(1024, MODE == kGatherRpie || MODE == kGatherBl
     }
   }
   const size_t o = (size_t)y * a.nxo + x;
-  if (MODE == kGatherOverlap || MODE == kGatherBlend) {
+  if (MODE == kGatherRpie || MODE == kGatherBlend) {
     float d = 0.f;
 #pragma unroll
     for (int m = 0; m < kMaxModes; ++m)
@@ -185,6 +183,15 @@ __global__ void __launch_bounds__(1024, MODE == kGatherRpie || MODE == kGatherBl
       // psi_to_obj_probe's object sums (engine/ops.rs:352-369), every pixel, covered or not
       a.out[o] = num[0].value();
       a.pre[o] = d;
+    }
+    if (MODE == kGatherRpie && inside && grp == 0) {
+      const size_t no = (size_t)a.nyo * a.nxo;
+#pragma unroll
+      for (int m = 0; m < kMaxModes; ++m) {
+        if (m >= K) break;
+        a.out[m * no + o] = num[m].value();
+        a.pre[m * no + o] = covered ? den[m].s : -1.f;
+      }
     }
     d = warp_max(inside && grp == 0 ? d : 0.f);
     if (threadIdx.x % 32 == 0) red[threadIdx.x / 32] = d;
@@ -197,18 +204,7 @@ __global__ void __launch_bounds__(1024, MODE == kGatherRpie || MODE == kGatherBl
     return;
   }
   if (!inside || grp != 0) return;
-  if (MODE == kGatherRpie) {
-    if (!covered) return;
-    const float pmax = *a.pmax;
-    float2 d = make_float2(0.f, 0.f);
-#pragma unroll
-    for (int m = 0; m < kMaxModes; ++m) {
-      if (m >= K) break;
-      const float w = (1.f - a.alpha) * den[m].s + a.alpha * pmax;
-      d = cadd(d, cscale(num[m].value(), 1.f / w));
-    }
-    a.object[o] = cadd(a.object[o], cscale(d, a.step));
-  } else if (MODE == kGatherLsqml) {
+  if (MODE == kGatherLsqml) {
     const float p = a.pre[o];
     const float fl = 0.1f * (*a.pre_max);
     a.out[o] = cscale(num[0].value(), rsqrtf(p * p + fl * fl));
@@ -230,6 +226,29 @@ __global__ void __launch_bounds__(1024, MODE == kGatherRpie || MODE == kGatherBl
     // pty-chi's schedule: (pre + I)/2, the first from pre = I·pre_scale.
     a.pre[o] = a.pre_scale >= 0.f ? 0.5f * (d * a.pre_scale + d) : 0.5f * (a.pre[o] + d);
   }
+}
+
+template <int MODE>
+static __global__ void __launch_bounds__(1024, MODE == kGatherBlend ? 1 : 2)
+    object_tile_kernel(GatherArgs a) {
+  object_tile<MODE>(a);
+}
+
+// Σ over `n` planes of `count` values at value i, in plane order, compensated; ten loads ahead of
+// the additions (they alone took 7 of a 64² batch's 10.6 us with the loads one by one).
+PTYB_D float2 plane_sum(const float2* planes, int n, int count, int i) {
+  KahanC acc;
+  acc.init();
+  int ch = 0;
+  for (; ch + 10 <= n; ch += 10) {
+    float2 v[10];
+#pragma unroll
+    for (int k = 0; k < 10; ++k) v[k] = planes[(size_t)(ch + k) * count + i];
+#pragma unroll
+    for (int k = 0; k < 10; ++k) acc.add(v[k]);
+  }
+  for (; ch < n; ++ch) acc.add(planes[(size_t)ch * count + i]);
+  return acc.value();
 }
 
 struct ProbeArgs {
@@ -314,6 +333,88 @@ static __global__ void __launch_bounds__(256) probe_partial_kernel(ProbeArgs a) 
   if (a.mode >= 2)
     reinterpret_cast<float2*>(a.partial_den + (size_t)blockIdx.y * plane)[pix / 2] =
         make_float2(den[0].s - den[0].c, den[1].s - den[1].c);
+}
+
+// rPIE's object sums (the first `ntiles` blocks, one object tile each) and probe sums (the rest:
+// 1024 pixels of one chunk of slots, one pixel a thread, mode 0's weight) of a batch in one
+// launch. Both read the batch-start object and probe, and at 64² neither fills the GPU: the
+// tiles of a 256² object 256 of its SMs' 296 places, each for the latency of a few views. With
+// the maximum of the overlaps taken here and the updates in rpie_apply_kernel a batch is three
+// launches instead of five: frame pass, sums, updates.
+static __global__ void __launch_bounds__(1024, 1) rpie_sums_kernel(GatherArgs g, ProbeArgs a,
+                                                                   int ntiles) {
+  if (blockIdx.x < ntiles) {
+    object_tile<kGatherRpie>(g);
+    return;
+  }
+  __shared__ int2 cs[kMaxProbeChunk];
+  __shared__ float om[kMaxProbeChunk];
+  const int N = a.N, blocks = N * N / 1024, block = blockIdx.x - ntiles;
+  const int chunk = block / blocks;
+  const size_t plane = (size_t)N * N;
+  const int s0 = chunk * a.chunk, s1 = min(a.nslot, s0 + a.chunk);
+  for (int i = threadIdx.x; i < s1 - s0; i += 1024) {
+    cs[i] = a.corners[a.frames[s0 + i]];
+    om[i] = a.omax[s0 + i];
+  }
+  __syncthreads();
+  const int pix = (block % blocks) * 1024 + threadIdx.x;
+  const float2 q = a.quad[pix];
+  const float2* obj = a.object + (size_t)(pix / N) * a.nxo + pix % N;
+  KahanC acc[kMaxModes];
+#pragma unroll
+  for (int m = 0; m < kMaxModes; ++m) acc[m].init();
+#pragma unroll 2
+  for (int s = s0; s < s1; ++s) {
+    const int2 c = cs[s - s0];
+    const float2 o = obj[(size_t)c.x * a.nxo + c.y];
+    float2 w = cconj(cmul(o, q));
+    w = cscale(w, 1.f / ((1.f - a.alpha) * cnorm2(o) + a.alpha * om[s - s0]));
+#pragma unroll
+    for (int m = 0; m < kMaxModes; ++m) {
+      if (m >= a.K) break;
+      acc[m].add(cmul(w, a.upd[((size_t)s * a.K + m) * plane + pix]));
+    }
+  }
+#pragma unroll
+  for (int m = 0; m < kMaxModes; ++m)
+    if (m < a.K) a.partial[((size_t)chunk * a.K + m) * plane + pix] = acc[m].value();
+}
+
+// rPIE's updates of a batch in one launch: the first `oblocks` blocks take the object,
+// O += step·Σ_m num_m / ((1−α)·D_m + α·pmax) on covered pixels, the rest the probe,
+// P += coef·Σ over the `nsum` planes in order. `pmax_next` is cleared for the batch that follows.
+struct RpieApplyArgs {
+  float2* object;
+  const float2* num;  // [K][no]
+  const float* den;   // [K][no], < 0 where no view covers the pixel
+  const float* pmax;
+  float* pmax_next;
+  float2* probe;
+  const float2* sums; // [nsum][count]
+  size_t no;
+  int K, nsum, count, oblocks;
+  float alpha, step, coef;
+};
+static __global__ void __launch_bounds__(256) rpie_apply_kernel(RpieApplyArgs a) {
+  if (blockIdx.x == 0 && threadIdx.x == 0) *a.pmax_next = 0.f;
+  if (blockIdx.x < a.oblocks) {
+    const size_t o = (size_t)blockIdx.x * 256 + threadIdx.x;
+    if (o >= a.no || a.den[o] < 0.f) return;
+    const float pmax = *a.pmax;
+    float2 d = make_float2(0.f, 0.f);
+#pragma unroll
+    for (int m = 0; m < kMaxModes; ++m) {
+      if (m >= a.K) break;
+      const float w = (1.f - a.alpha) * a.den[m * a.no + o] + a.alpha * pmax;
+      d = cadd(d, cscale(a.num[m * a.no + o], 1.f / w));
+    }
+    a.object[o] = cadd(a.object[o], cscale(d, a.step));
+    return;
+  }
+  const int i = (blockIdx.x - a.oblocks) * 256 + threadIdx.x;
+  if (i >= a.count) return;
+  a.probe[i] = cadd(a.probe[i], cscale(plane_sum(a.sums, a.nsum, a.count, i), a.coef));
 }
 
 // One launch over `nchunk` chunks (K ≤ 4; N² is a multiple of 512 at every side).
@@ -446,10 +547,7 @@ static __global__ void probe_finalize_kernel(const float2* partial, int nchunk, 
                                       const float* norm_max = nullptr, int plane = 1) {
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= count) return;
-  KahanC acc;
-  acc.init();
-  for (int ch = 0; ch < nchunk; ++ch) acc.add(partial[(size_t)ch * count + i]);
-  const float2 v = acc.value();
+  const float2 v = plane_sum(partial, nchunk, count, i);
   if (mode == 0) {
     probe[i] = cadd(probe[i], cscale(v, coef));
   } else if (mode == 3) {

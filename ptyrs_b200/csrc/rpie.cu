@@ -8,8 +8,12 @@ using namespace ptyb;
 namespace ptyb::eng {
 namespace {
 
-// One rPIE batch (engine/ptycho.rs:904-1085; GPU launch sequence engine/gpu/rpie.rs:239-345).
-void rpie_batch(ptyb_handle* h, const ptyb_rpie_params& p, const int* frames, int nslot) {
+// One rPIE batch (engine/ptycho.rs:904-1085; GPU launch sequence engine/gpu/rpie.rs:239-345):
+// the frame pass, the object and probe sums from the batch-start arrays, the position model's
+// passes, then both updates. `pmax` and `pmax_next` take the largest overlap of this batch and
+// of the next in turn (h->rpie_max), each cleared by the updates of the batch before.
+void rpie_batch(ptyb_handle* h, const ptyb_rpie_params& p, const int* frames, int nslot,
+                float* pmax, float* pmax_next) {
   FrameArgs a = frame_args(h, frames);
   GatherArgs g = gather_args(h, frames, nslot);
   const int pstride = h->K * h->N * h->N;
@@ -27,36 +31,16 @@ void rpie_batch(ptyb_handle* h, const ptyb_rpie_params& p, const int* frames, in
   }
   check(h, launch_frame<kRpie>(h, a, nslot), "rpie frame pass");
   ++h->launches;
-  if (p.update_object) {
-    check(h, cudaMemsetAsync(h->scal, 0, sizeof(float), h->stream), "memset");
-    timed(h, kKObjOverlap, [&] { object_tile_kernel<kGatherOverlap><<<ntiles(h), 1024, 0, h->stream>>>(g); }, nslot);
-    launched(h, "overlap max");
-  }
-  if (refine) {
-    // pty-chi's position sums from mode 0 of the batch-start state (engine/ptycho.rs:1037-1064)
-    check(h, launch_move<kDerivWindow>(h, move_args(h, frames, h->field), nslot), "window derivative");
-    ++h->launches;
-    timed(h, kKPositionSums, [&] {
-      position_sums_kernel<<<nslot, 256, 0, h->stream>>>(h->field, h->wave, pstride, h->quad,
-                                                          h->upd, h->K, h->N, h->pos_sums);
-    }, nslot);
-    launched(h, "position sums");
-  }
   const int count = h->K * h->N * h->N;
+  // the probe's plain sums run beside the object's; under the move its directions go back first
+  const bool sum_probe = p.update_probe && !moved;
   int nchunk = 0;
-  if (p.update_probe && moved) {
-    // each frame's rPIE probe direction moved back by −d (engine/ptycho.rs:1007-1035)
-    timed(h, kKProbePartial, [&] {
-      probe_terms_kernel<<<dim3((h->N * h->N + 255) / 256, nslot), 256, 0, h->stream>>>(
-          h->object, h->quad, h->upd, frames, h->corners, h->nxo, h->K, h->N, h->field, h->omax,
-          (float)p.probe_alpha);
-    }, nslot);
-    launched(h, "probe terms");
-    check(h, launch_move<kMoveBack>(h, move_args(h, frames, h->field), nslot), "probe move back");
-    ++h->launches;
-  } else if (p.update_probe) {
-    // Reads the batch-start object, so it runs before the object update.
-    const int chunk = probe_chunk(h, nslot, &nchunk);
+  const int chunk = sum_probe ? probe_chunk(h, nslot, &nchunk) : 0;
+  const int tiles = p.update_object ? ntiles(h) : 0, pblocks = nchunk * (h->N * h->N / 1024);
+  if (tiles + pblocks > 0) {
+    g.out = h->rpie_num;
+    g.pre = h->rpie_den;
+    g.pmax = pmax;
     ProbeArgs pa = {};
     pa.object = h->object;
     pa.quad = h->quad;
@@ -71,24 +55,52 @@ void rpie_batch(ptyb_handle* h, const ptyb_rpie_params& p, const int* frames, in
     pa.nxo = h->nxo;
     pa.K = h->K;
     pa.N = h->N;
-    pa.mode = 0;
-    timed(h, kKProbePartial, [&] { launch_probe_partial(pa, nchunk, h->stream); }, pa.nslot);
-    launched(h, "probe partial");
+    timed(h, kKObjRpie, [&] { rpie_sums_kernel<<<tiles + pblocks, 1024, 0, h->stream>>>(g, pa, tiles); }, nslot);
+    launched(h, "rpie sums");
   }
-  if (p.update_object) {
-    g.alpha = (float)p.obj_alpha;
-    g.step = (float)p.obj_step;
-    timed(h, kKObjRpie, [&] { object_tile_kernel<kGatherRpie><<<ntiles(h), 1024, 0, h->stream>>>(g); }, g.nslot);
-    launched(h, "object update");
+  if (refine) {
+    // pty-chi's position sums from mode 0 of the batch-start state (engine/ptycho.rs:1037-1064)
+    check(h, launch_move<kDerivWindow>(h, move_args(h, frames, h->field), nslot), "window derivative");
+    ++h->launches;
+    timed(h, kKPositionSums, [&] {
+      position_sums_kernel<<<nslot, 256, 0, h->stream>>>(h->field, h->wave, pstride, h->quad,
+                                                          h->upd, h->K, h->N, h->pos_sums);
+    }, nslot);
+    launched(h, "position sums");
   }
-  if (p.update_probe) {
-    // P += step/nbatch · Σ (frames in order); the gathers above read the batch-start probe
+  if (p.update_probe && moved) {
+    // each frame's rPIE probe direction moved back by −d (engine/ptycho.rs:1007-1035)
+    timed(h, kKProbePartial, [&] {
+      probe_terms_kernel<<<dim3((h->N * h->N + 255) / 256, nslot), 256, 0, h->stream>>>(
+          h->object, h->quad, h->upd, frames, h->corners, h->nxo, h->K, h->N, h->field, h->omax,
+          (float)p.probe_alpha);
+    }, nslot);
+    launched(h, "probe terms");
+    check(h, launch_move<kMoveBack>(h, move_args(h, frames, h->field), nslot), "probe move back");
+    ++h->launches;
+  }
+  // O and P += step/nbatch · Σ (frames in order)
+  RpieApplyArgs u = {};
+  u.object = h->object;
+  u.num = h->rpie_num;
+  u.den = h->rpie_den;
+  u.pmax = pmax;
+  u.pmax_next = pmax_next;
+  u.probe = h->probe;
+  u.sums = moved ? h->field : h->partial;
+  u.no = (size_t)h->nyo * h->nxo;
+  u.K = h->K;
+  u.nsum = moved ? nslot : nchunk;
+  u.count = p.update_probe ? count : 0;
+  u.oblocks = p.update_object ? (int)blocks_for(u.no) : 0;
+  u.alpha = (float)p.obj_alpha;
+  u.step = (float)p.obj_step;
+  u.coef = (float)(p.probe_step / nslot);
+  if (u.oblocks + u.count > 0) {
     timed(h, kKProbeFinal, [&] {
-      probe_finalize_kernel<<<(count + 255) / 256, 256, 0, h->stream>>>(
-          moved ? h->field : h->partial, moved ? nslot : nchunk, count, h->probe, nullptr,
-          nullptr, (float)(p.probe_step / nslot), 0);
+      rpie_apply_kernel<<<u.oblocks + blocks_for(u.count), 256, 0, h->stream>>>(u);
     });
-    launched(h, "probe update");
+    launched(h, "rpie updates");
   }
   if (refine) {
     const double eps = 1e-6 * ((double)h->N * h->N);
@@ -126,13 +138,22 @@ int ptyb_rpie(ptyb_handle* h, const ptyb_rpie_params* p, int32_t nepoch) {
     ensure_slots(h, std::max(bs, std::min(h->P, h->stack)));
     std::vector<std::vector<int32_t>> sizes;
     upload_orders(h, nepoch, p->batch_size, p->seed, h->cycle, &sizes, nullptr);
+    if (!h->rpie_num) {
+      const size_t no = (size_t)h->nyo * h->nxo;
+      h->rpie_num = alloc<float2>(h, h->K * no);
+      h->rpie_den = alloc<float>(h, h->K * no);
+      h->rpie_max = alloc<float>(h, 2);
+    }
     begin_call(h);
+    check(h, cudaMemsetAsync(h->rpie_max, 0, 2 * sizeof(float), h->stream), "memset");
+    int64_t batch = 0;
     for (int ic = 0; ic < nepoch; ++ic) {
       const int* order = h->order_all + (size_t)ic * h->P;
       int off = 0;
       for (int n : sizes[ic]) {
-        rpie_batch(h, *p, order + off, n);
+        rpie_batch(h, *p, order + off, n, h->rpie_max + batch % 2, h->rpie_max + (batch + 1) % 2);
         off += n;
+        ++batch;
       }
       if (llk_due(p->calc_llk, ic, nepoch)) record(h, kAlgRpie, llk_pass(h));
       ++h->cycle;
