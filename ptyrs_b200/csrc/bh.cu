@@ -61,7 +61,7 @@ void bh_grads(ptyb_handle* h, const int* frames, int n) {
       g.probe = h->wave;
       g.probe_stride = (int)np;
     }
-    timed(h, kKObjMl, [&] { object_tile_kernel<kGatherMl><<<ntiles(h), 1024, 0, h->stream>>>(g); }, m);
+    timed(h, kKObjMl, [&] { launch_object_tiles<kGatherMl>(g, ntiles(h), h->stream); }, m);
     launched(h, "bh object gradient");
     if (pos) {
       // DFT(conj(O_win)·g)·exp(+2πi f·d) per frame, summed in frame order (the moves' adjoint)

@@ -62,7 +62,7 @@ void object_blend(ptyb_handle* h, double inertia, const float2* waves = nullptr)
   g.out = h->d_obj;
   g.pre = h->blend_norm;
   check(h, cudaMemsetAsync(g.pmax, 0, sizeof(float), h->stream), "memset");
-  timed(h, kKObjBlend, [&] { object_tile_kernel<kGatherBlend><<<ntiles(h), 1024, 0, h->stream>>>(g); }, h->P);
+  timed(h, kKObjBlend, [&] { launch_object_tiles<kGatherBlend>(g, ntiles(h), h->stream); }, h->P);
   launched(h, "object blend sums");
   const size_t no = (size_t)h->nyo * h->nxo;
   timed(h, kKAxpy, [&] {

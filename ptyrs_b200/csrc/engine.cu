@@ -350,7 +350,7 @@ GatherArgs gather_args(ptyb_handle* h, const int* frames, int nslot) {
 }
 
 int ntiles(ptyb_handle* h) {
-  return ((h->nyo + kTile - 1) / kTile) * ((h->nxo + kTile - 1) / kTile);
+  return ((h->nyo + kTileRows - 1) / kTileRows) * ((h->nxo + kTile - 1) / kTile);
 }
 
 // Scratch for `n` frames per launch.

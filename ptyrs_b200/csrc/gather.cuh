@@ -1,19 +1,21 @@
 // Deterministic scatter-adds of the per-view updates onto the object and the probe.
 //
-// Object: one CTA owns a 16×16 object tile and lists the launch's views that overlap it in
-// ascending slot order (the reference's view order); four thread groups per pixel take every
-// fourth view of that list, each with Kahan-compensated float sums, and the groups' sums are
-// added in group order. No atomics touch the object and the result does not depend on
+// Object: one CTA owns half of a 16×16 square of the object and lists the launch's views that
+// overlap the square in ascending slot order (the reference's view order); four thread groups
+// per pixel take every fourth view of that list, each with Kahan-compensated float sums, and the
+// groups' sums are added in group order. No atomics touch the object and the result does not depend on
 // scheduling (the reference's tile-owned gather, ptyrs-kernels/src/lib.rs:388-437; operator
 // engine/ops.rs:282-310). Probe: the slots are cut
-// into chunks, each CTA sums one chunk in slot order for 256 probe pixels, and a second pass
+// into chunks, each CTA sums one chunk in slot order for 512 probe pixels, and a second pass
 // adds the chunk sums in chunk order (engine/ops.rs:315-345).
 #pragma once
 #include "common.cuh"
 
 namespace ptyb {
 
-constexpr int kTile = 16;      // object tile side
+constexpr int kTile = 16;      // object tile width
+constexpr int kTileThreads = 512;                    // threads of a tile's CTA
+constexpr int kTileRows = kTileThreads / 4 / kTile;  // object tile height (kGroups threads a pixel)
 constexpr int kGroups = 4;     // view groups per pixel
 constexpr int kMaxModes = 4;
 
@@ -42,9 +44,9 @@ struct GatherArgs {
   int probe_stride;        // elements between slots' probes (0: the shared probe)
 };
 
-// The launch's slots in [s0, s1) (at most 1024) whose window overlaps the tile
-// [ty0, ty0+16) × [tx0, tx0+16), in ascending order with their corners: an ordered
-// compaction by all 1024 threads (warp ballots, then a prefix over the warps).
+// The launch's slots in [s0, s1) (at most kTileThreads) whose window overlaps the square
+// [ty0, ty0 + kTile) × [tx0, tx0 + kTile), in ascending order with their corners: an ordered
+// compaction by the whole CTA (warp ballots, then a prefix over the warps).
 PTYB_D int tile_list(const GatherArgs& a, int s0, int s1, int ty0, int tx0, int* list,
                      int2* corner) {
   __shared__ int wbase[32];
@@ -61,7 +63,7 @@ PTYB_D int tile_list(const GatherArgs& a, int s0, int s1, int ty0, int tx0, int*
   if (lane == 0) wbase[w] = __popc(m);
   __syncthreads();
   if (w == 0) {
-    const int v = wbase[lane];
+    const int v = lane < kTileThreads / 32 ? wbase[lane] : 0;
     int incl = v;
 #pragma unroll
     for (int o = 1; o < 32; o <<= 1) {
@@ -83,70 +85,78 @@ PTYB_D int tile_list(const GatherArgs& a, int s0, int s1, int ty0, int tx0, int*
   return n;
 }
 
-template <int MODE>
+// One tile of the object for a launch of K probe modes: every group of threads walks its
+// views in order, `kAhead` of them at a time: their loads are all issued before the first is
+// added. K is a template parameter so that a view costs the registers its modes need.
+template <int MODE, int K>
 PTYB_D void object_tile(const GatherArgs& a) {
-  constexpr int kChunk = 1024;
-  constexpr int kPix = kTile * kTile;  // 256 pixels, kGroups threads each
+  constexpr int kChunk = kTileThreads;
+  constexpr int kPix = kTile * kTileRows;  // pixels, kGroups threads each
+  constexpr int kAhead = K <= 2 ? 2 : 1;
+  constexpr bool kNum = MODE != kGatherIllum;
+  constexpr bool kDen = MODE == kGatherIllum || MODE == kGatherRpie || MODE == kGatherBlend;
+  constexpr int NM = MODE == kGatherRpie ? K : 1;  // numerators kept apart
+  constexpr int DM = kDen ? K : 1;
   // The view list (during the walk), then the groups' partial sums (after it).
   constexpr int kListBytes = kChunk * (sizeof(int) + sizeof(int2));
-  constexpr int kNumBytes = (kGroups - 1) * kMaxModes * kPix * sizeof(float2);
-  constexpr int kDenBytes = (kGroups - 1) * kMaxModes * kPix * sizeof(float);
+  constexpr int kNumBytes = (kGroups - 1) * NM * kPix * sizeof(float2);
+  constexpr int kDenBytes = (kGroups - 1) * DM * kPix * sizeof(float);
   constexpr int kPartBytes = kNumBytes + kDenBytes + (kGroups - 1) * kPix * sizeof(int);
   __shared__ __align__(16) unsigned char sm[kListBytes > kPartBytes ? kListBytes : kPartBytes];
   __shared__ float red[32];
   int* list = reinterpret_cast<int*>(sm);
   int2* lcorner = reinterpret_cast<int2*>(sm + kChunk * sizeof(int));
-  float2(*part_num)[kMaxModes][kPix] = reinterpret_cast<float2(*)[kMaxModes][kPix]>(sm);
-  float(*part_den)[kMaxModes][kPix] = reinterpret_cast<float(*)[kMaxModes][kPix]>(sm + kNumBytes);
+  float2(*part_num)[NM][kPix] = reinterpret_cast<float2(*)[NM][kPix]>(sm);
+  float(*part_den)[DM][kPix] = reinterpret_cast<float(*)[DM][kPix]>(sm + kNumBytes);
   int(*part_cov)[kPix] = reinterpret_cast<int(*)[kPix]>(sm + kNumBytes + kDenBytes);
   const int tiles_x = (a.nxo + kTile - 1) / kTile;
-  const int tx0 = (blockIdx.x % tiles_x) * kTile, ty0 = (blockIdx.x / tiles_x) * kTile;
+  const int tx0 = (blockIdx.x % tiles_x) * kTile, ty0 = (blockIdx.x / tiles_x) * kTileRows;
   const int px = threadIdx.x % kPix, grp = threadIdx.x / kPix;
   const int x = tx0 + px % kTile, y = ty0 + px / kTile;
   const bool inside = x < a.nxo && y < a.nyo;
-  const int K = a.nprobe;
   const int N = a.N;
   const size_t plane = (size_t)N * N;
-  KahanC num[kMaxModes];
-  Kahan den[kMaxModes];
+  KahanC num[NM];
+  Kahan den[DM];
 #pragma unroll
-  for (int m = 0; m < kMaxModes; ++m) {
-    num[m].init();
-    den[m].init();
-  }
+  for (int m = 0; m < NM; ++m) num[m].init();
+#pragma unroll
+  for (int m = 0; m < DM; ++m) den[m].init();
   bool covered = false, any = false;
   for (int s0 = 0; s0 < a.nslot; s0 += kChunk) {
     const int s1 = min(a.nslot, s0 + kChunk);
-    const int n = tile_list(a, s0, s1, ty0, tx0, list, lcorner);
+    const int n = tile_list(a, s0, s1, ty0 & ~(kTile - 1), tx0, list, lcorner);
     any |= n > 0;
-#pragma unroll 2
-    for (int i = grp; i < n; i += kGroups) {
-      const int s = list[i];
-      const int2 c = lcorner[i];
-      const int yy = y - c.x, xx = x - c.y;
-      if (!inside || yy < 0 || yy >= N || xx < 0 || xx >= N) continue;
-      covered = true;
-      const int pix = yy * N + xx;
-      const float2 q = a.quad[pix];
-      float2 u[kMaxModes];
+    for (int i0 = grp; i0 < n; i0 += kGroups * kAhead) {
+      bool ok[kAhead];
+      float2 q[kAhead], u[kAhead][K], p[kAhead][K];
 #pragma unroll
-      for (int m = 0; m < kMaxModes; ++m)
-        if (m < K && (MODE == kGatherRpie || MODE == kGatherLsqml || MODE == kGatherMl ||
-                      MODE == kGatherBlend))
-          u[m] = a.upd[((size_t)s * K + m) * plane + pix];
+      for (int j = 0; j < kAhead; ++j) {
+        const int i = i0 + j * kGroups;
+        ok[j] = false;
+        if (i >= n) continue;
+        const int s = list[i];
+        const int2 c = lcorner[i];
+        const int yy = y - c.x, xx = x - c.y;
+        ok[j] = inside && yy >= 0 && yy < N && xx >= 0 && xx < N;
+        if (!ok[j]) continue;
+        const int pix = yy * N + xx;
+        if (kNum) q[j] = a.quad[pix];
 #pragma unroll
-      for (int m = 0; m < kMaxModes; ++m) {
-        if (m >= K) break;
-        const float2 p = a.probe[(size_t)s * a.probe_stride + m * plane + pix];
-        if (MODE == kGatherIllum || MODE == kGatherRpie || MODE == kGatherBlend)
-          den[m].add(cnorm2(p));
-        if (MODE == kGatherRpie || MODE == kGatherLsqml || MODE == kGatherMl ||
-            MODE == kGatherBlend) {
-          const float2 t = cmulc(cmul(p, q), u[m]);  // conj(P·q)·u
-          if (MODE == kGatherRpie)
-            num[m].add(t);
-          else
-            num[0].add(t);
+        for (int m = 0; m < K; ++m) {
+          if (kNum) u[j][m] = a.upd[((size_t)s * K + m) * plane + pix];
+          p[j][m] = a.probe[(size_t)s * a.probe_stride + m * plane + pix];
+        }
+      }
+#pragma unroll
+      for (int j = 0; j < kAhead; ++j) {
+        if (!ok[j]) continue;
+        covered = true;
+#pragma unroll
+        for (int m = 0; m < K; ++m) {
+          if (kDen) den[m].add(cnorm2(p[j][m]));
+          // conj(P·q)·u
+          if (kNum) num[NM == 1 ? 0 : m].add(cmulc_rn(cmul_rn(p[j][m], q[j]), u[j][m]));
         }
       }
     }
@@ -155,10 +165,10 @@ PTYB_D void object_tile(const GatherArgs& a) {
   __syncthreads();  // the list's space becomes the partial sums'
   if (grp > 0) {
 #pragma unroll
-    for (int m = 0; m < kMaxModes; ++m) {
+    for (int m = 0; m < NM; ++m)
       part_num[grp - 1][m][px] = make_float2(num[m].re.s - num[m].re.c, num[m].im.s - num[m].im.c);
-      part_den[grp - 1][m][px] = den[m].s - den[m].c;
-    }
+#pragma unroll
+    for (int m = 0; m < DM; ++m) part_den[grp - 1][m][px] = den[m].s - den[m].c;
     part_cov[grp - 1][px] = covered;
   }
   __syncthreads();
@@ -166,10 +176,9 @@ PTYB_D void object_tile(const GatherArgs& a) {
 #pragma unroll
     for (int g = 0; g < kGroups - 1; ++g) {
 #pragma unroll
-      for (int m = 0; m < kMaxModes; ++m) {
-        num[m].add(part_num[g][m][px]);
-        den[m].add(part_den[g][m][px]);
-      }
+      for (int m = 0; m < NM; ++m) num[m].add(part_num[g][m][px]);
+#pragma unroll
+      for (int m = 0; m < DM; ++m) den[m].add(part_den[g][m][px]);
       covered |= part_cov[g][px] != 0;
     }
   }
@@ -177,8 +186,7 @@ PTYB_D void object_tile(const GatherArgs& a) {
   if (MODE == kGatherRpie || MODE == kGatherBlend) {
     float d = 0.f;
 #pragma unroll
-    for (int m = 0; m < kMaxModes; ++m)
-      if (m < K) d += den[m].s;
+    for (int m = 0; m < DM; ++m) d += den[m].s;
     if (MODE == kGatherBlend && inside && grp == 0) {
       // psi_to_obj_probe's object sums (engine/ops.rs:352-369), every pixel, covered or not
       a.out[o] = num[0].value();
@@ -187,8 +195,7 @@ PTYB_D void object_tile(const GatherArgs& a) {
     if (MODE == kGatherRpie && inside && grp == 0) {
       const size_t no = (size_t)a.nyo * a.nxo;
 #pragma unroll
-      for (int m = 0; m < kMaxModes; ++m) {
-        if (m >= K) break;
+      for (int m = 0; m < NM; ++m) {
         a.out[m * no + o] = num[m].value();
         a.pre[m * no + o] = covered ? den[m].s : -1.f;
       }
@@ -198,7 +205,7 @@ PTYB_D void object_tile(const GatherArgs& a) {
     __syncthreads();
     if (threadIdx.x == 0) {
       float mx = 0.f;
-      for (int w = 0; w < 32; ++w) mx = fmaxf(mx, red[w]);
+      for (int w = 0; w < kTileThreads / 32; ++w) mx = fmaxf(mx, red[w]);
       atomic_max_nonneg(a.pmax, mx);
     }
     return;
@@ -221,17 +228,38 @@ PTYB_D void object_tile(const GatherArgs& a) {
   } else if (MODE == kGatherIllum) {
     float d = 0.f;
 #pragma unroll
-    for (int m = 0; m < kMaxModes; ++m)
-      if (m < K) d += den[m].s;
+    for (int m = 0; m < DM; ++m) d += den[m].s;
     // pty-chi's schedule: (pre + I)/2, the first from pre = I·pre_scale.
     a.pre[o] = a.pre_scale >= 0.f ? 0.5f * (d * a.pre_scale + d) : 0.5f * (a.pre[o] + d);
   }
 }
 
-template <int MODE>
-static __global__ void __launch_bounds__(1024, MODE == kGatherBlend ? 1 : 2)
+// CTAs of 512 threads per SM a tile kernel is compiled for, by what a thread holds: 42 registers
+// for two views of up to two modes (ML 256² x 2 0.538 -> 0.460 us per frame, blend 0.477 -> 0.376,
+// 128² x 1 0.106 -> 0.071, against CTAs of 1024 with the mode count at run time; 64 registers
+// took 0.511, 0.375 and 0.077), 64 for rPIE's sums per mode of two modes and more (128² x 2 0.39
+// -> 0.29; at one mode 42 are ahead, 0.127 to 0.146), 32 for one view of three or four modes
+// (LSQML 128² x 3 0.265; 0.322 at 42 with two views).
+template <int MODE, int K>
+__host__ __device__ constexpr int tile_min_blocks() {
+  return MODE == kGatherRpie ? (K == 1 ? 3 : 2) : K <= 2 || MODE == kGatherBlend ? 3 : 4;
+}
+
+template <int MODE, int K>
+static __global__ void __launch_bounds__(kTileThreads, tile_min_blocks<MODE, K>())
     object_tile_kernel(GatherArgs a) {
-  object_tile<MODE>(a);
+  object_tile<MODE, K>(a);
+}
+
+// One launch of a.nprobe ≤ 4 modes over `tiles` object tiles.
+template <int MODE>
+static inline void launch_object_tiles(const GatherArgs& a, int tiles, cudaStream_t s) {
+  switch (a.nprobe) {
+    case 1: object_tile_kernel<MODE, 1><<<tiles, kTileThreads, 0, s>>>(a); break;
+    case 2: object_tile_kernel<MODE, 2><<<tiles, kTileThreads, 0, s>>>(a); break;
+    case 3: object_tile_kernel<MODE, 3><<<tiles, kTileThreads, 0, s>>>(a); break;
+    default: object_tile_kernel<MODE, 4><<<tiles, kTileThreads, 0, s>>>(a);
+  }
 }
 
 // Σ over `n` planes of `count` values at value i, in plane order, compensated; ten loads ahead of
@@ -336,34 +364,35 @@ static __global__ void __launch_bounds__(256) probe_partial_kernel(ProbeArgs a) 
 }
 
 // rPIE's object sums (the first `ntiles` blocks, one object tile each) and probe sums (the rest:
-// 1024 pixels of one chunk of slots, one pixel a thread, mode 0's weight) of a batch in one
-// launch. Both read the batch-start object and probe, and at 64² neither fills the GPU: the
-// tiles of a 256² object 256 of its SMs' 296 places, each for the latency of a few views. With
-// the maximum of the overlaps taken here and the updates in rpie_apply_kernel a batch is three
-// launches instead of five: frame pass, sums, updates.
-static __global__ void __launch_bounds__(1024, 1) rpie_sums_kernel(GatherArgs g, ProbeArgs a,
-                                                                   int ntiles) {
+// kTileThreads pixels of one chunk of slots, one a thread, mode 0's weight) of a batch in one
+// launch. Both read the batch-start object and probe, and at 64² neither fills the GPU for more
+// than the latency of a few views. With the maximum of the overlaps taken here and the updates in
+// rpie_apply_kernel a batch is three launches instead of five: frame pass, sums, updates (46 ->
+// 28 us for 100 frames of 64²).
+template <int K>
+static __global__ void __launch_bounds__(kTileThreads, tile_min_blocks<kGatherRpie, K>())
+    rpie_sums_kernel(GatherArgs g, ProbeArgs a, int ntiles) {
   if (blockIdx.x < ntiles) {
-    object_tile<kGatherRpie>(g);
+    object_tile<kGatherRpie, K>(g);
     return;
   }
   __shared__ int2 cs[kMaxProbeChunk];
   __shared__ float om[kMaxProbeChunk];
-  const int N = a.N, blocks = N * N / 1024, block = blockIdx.x - ntiles;
+  const int N = a.N, blocks = N * N / kTileThreads, block = blockIdx.x - ntiles;
   const int chunk = block / blocks;
   const size_t plane = (size_t)N * N;
   const int s0 = chunk * a.chunk, s1 = min(a.nslot, s0 + a.chunk);
-  for (int i = threadIdx.x; i < s1 - s0; i += 1024) {
+  for (int i = threadIdx.x; i < s1 - s0; i += kTileThreads) {
     cs[i] = a.corners[a.frames[s0 + i]];
     om[i] = a.omax[s0 + i];
   }
   __syncthreads();
-  const int pix = (block % blocks) * 1024 + threadIdx.x;
+  const int pix = (block % blocks) * kTileThreads + threadIdx.x;
   const float2 q = a.quad[pix];
   const float2* obj = a.object + (size_t)(pix / N) * a.nxo + pix % N;
-  KahanC acc[kMaxModes];
+  KahanC acc[K];
 #pragma unroll
-  for (int m = 0; m < kMaxModes; ++m) acc[m].init();
+  for (int m = 0; m < K; ++m) acc[m].init();
 #pragma unroll 2
   for (int s = s0; s < s1; ++s) {
     const int2 c = cs[s - s0];
@@ -371,14 +400,20 @@ static __global__ void __launch_bounds__(1024, 1) rpie_sums_kernel(GatherArgs g,
     float2 w = cconj(cmul(o, q));
     w = cscale(w, 1.f / ((1.f - a.alpha) * cnorm2(o) + a.alpha * om[s - s0]));
 #pragma unroll
-    for (int m = 0; m < kMaxModes; ++m) {
-      if (m >= a.K) break;
-      acc[m].add(cmul(w, a.upd[((size_t)s * a.K + m) * plane + pix]));
-    }
+    for (int m = 0; m < K; ++m) acc[m].add(cmul(w, a.upd[((size_t)s * K + m) * plane + pix]));
   }
 #pragma unroll
-  for (int m = 0; m < kMaxModes; ++m)
-    if (m < a.K) a.partial[((size_t)chunk * a.K + m) * plane + pix] = acc[m].value();
+  for (int m = 0; m < K; ++m) a.partial[((size_t)chunk * K + m) * plane + pix] = acc[m].value();
+}
+
+static inline void launch_rpie_sums(const GatherArgs& g, const ProbeArgs& a, int ntiles,
+                                    int blocks, cudaStream_t s) {
+  switch (g.nprobe) {
+    case 1: rpie_sums_kernel<1><<<blocks, kTileThreads, 0, s>>>(g, a, ntiles); break;
+    case 2: rpie_sums_kernel<2><<<blocks, kTileThreads, 0, s>>>(g, a, ntiles); break;
+    case 3: rpie_sums_kernel<3><<<blocks, kTileThreads, 0, s>>>(g, a, ntiles); break;
+    default: rpie_sums_kernel<4><<<blocks, kTileThreads, 0, s>>>(g, a, ntiles);
+  }
 }
 
 // rPIE's updates of a batch in one launch: the first `oblocks` blocks take the object,

@@ -30,7 +30,7 @@ void step_arrays(ptyb_handle* h, float2* obj, const float2* d_obj, int which, si
 void lsqml_preconditioner(ptyb_handle* h, bool init) {
   GatherArgs g = gather_args(h, h->iota, h->P);
   g.pre_scale = init ? (float)(h->max_power / (4.0 * h->N * h->N * ((double)h->N * h->N))) : -1.f;
-  timed(h, kKIllum, [&] { object_tile_kernel<kGatherIllum><<<ntiles(h), 1024, 0, h->stream>>>(g); });
+  timed(h, kKIllum, [&] { launch_object_tiles<kGatherIllum>(g, ntiles(h), h->stream); });
   launched(h, "illumination");
   check(h, cudaMemsetAsync(h->scal + 1, 0, sizeof(float), h->stream), "memset");
   const size_t n = (size_t)h->nyo * h->nxo;
@@ -127,7 +127,7 @@ void lsqml_batch_slices(ptyb_handle* h, const ptyb_lsqml_params& p, const int* f
       g.probe = own;
       g.probe_stride = (int)fplanes;
     }
-    timed(h, kKObjLsqml, [&] { object_tile_kernel<kGatherLsqml><<<ntiles(h), 1024, 0, h->stream>>>(g); }, nslot);
+    timed(h, kKObjLsqml, [&] { launch_object_tiles<kGatherLsqml>(g, ntiles(h), h->stream); }, nslot);
     launched(h, "slice object direction");
   }
   // probe direction from χ of slice 0 through slice 0's windows (no phase when S > 1)
@@ -345,7 +345,7 @@ void lsqml_batch(ptyb_handle* h, const ptyb_lsqml_params& p, const int* frames, 
     g.probe = own;
     g.probe_stride = pstride;
   }
-  timed(h, kKObjLsqml, [&] { object_tile_kernel<kGatherLsqml><<<ntiles(h), 1024, 0, h->stream>>>(g); }, nslot);
+  timed(h, kKObjLsqml, [&] { launch_object_tiles<kGatherLsqml>(g, ntiles(h), h->stream); }, nslot);
   launched(h, "object direction");
   const float2* dirs = nullptr;
   if (own)

@@ -56,7 +56,7 @@ void slice_gradients(ptyb_handle* h, bool uo, bool up, const int* frames_in, int
         g.probe = h->incident + (s - 1) * slice_stride;
         g.probe_stride = (int)fplanes;
       }
-      timed(h, kKObjMl, [&] { object_tile_kernel<kGatherMl><<<ntiles(h), 1024, 0, h->stream>>>(g); }, n);
+      timed(h, kKObjMl, [&] { launch_object_tiles<kGatherMl>(g, ntiles(h), h->stream); }, n);
       launched(h, "slice gradient");
     }
     if (up) {
@@ -151,7 +151,7 @@ void ml_gradients(ptyb_handle* h, bool uo, bool up, bool refine, bool pos_grad =
         g.probe = waves;
         g.probe_stride = pstride;
       }
-      timed(h, kKObjMl, [&] { object_tile_kernel<kGatherMl><<<ntiles(h), 1024, 0, h->stream>>>(g); }, n);
+      timed(h, kKObjMl, [&] { launch_object_tiles<kGatherMl>(g, ntiles(h), h->stream); }, n);
       launched(h, "object gradient");
     }
     if (up && h->have_offsets) {

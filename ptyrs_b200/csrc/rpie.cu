@@ -36,7 +36,7 @@ void rpie_batch(ptyb_handle* h, const ptyb_rpie_params& p, const int* frames, in
   const bool sum_probe = p.update_probe && !moved;
   int nchunk = 0;
   const int chunk = sum_probe ? probe_chunk(h, nslot, &nchunk) : 0;
-  const int tiles = p.update_object ? ntiles(h) : 0, pblocks = nchunk * (h->N * h->N / 1024);
+  const int tiles = p.update_object ? ntiles(h) : 0, pblocks = nchunk * (h->N * h->N / kTileThreads);
   if (tiles + pblocks > 0) {
     g.out = h->rpie_num;
     g.pre = h->rpie_den;
@@ -55,7 +55,7 @@ void rpie_batch(ptyb_handle* h, const ptyb_rpie_params& p, const int* frames, in
     pa.nxo = h->nxo;
     pa.K = h->K;
     pa.N = h->N;
-    timed(h, kKObjRpie, [&] { rpie_sums_kernel<<<tiles + pblocks, 1024, 0, h->stream>>>(g, pa, tiles); }, nslot);
+    timed(h, kKObjRpie, [&] { launch_rpie_sums(g, pa, tiles, tiles + pblocks, h->stream); }, nslot);
     launched(h, "rpie sums");
   }
   if (refine) {
