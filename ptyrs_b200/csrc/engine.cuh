@@ -101,7 +101,6 @@ struct ptyb_handle {
   double* pos_sums = nullptr;    // [slots][4]
   // Multislice (pty-chi's multislice object, LSQML only): slices, gap transfer functions, the
   // incident waves of slices 1.., every slice's χ, a plane of ones (slices without a phase).
-  int C_sums = 1;                // CTAs per frame of the position-sums transform
   int nslice = 1;
   float2* tf = nullptr;          // [nslice-1][N][N]
   float2* incident = nullptr;    // [nslice-1][slots][K][N][N]
@@ -300,9 +299,8 @@ cudaError_t launch_move(ptyb_handle* h, const MoveArgs& a, int nslot) {
                        : MODE == kSpectrum     ? kKSpectrum
                        : MODE == kBackSpectrum ? kKBackSpectrum
                                                : kKMove;
-  const int C = MODE == kDerivSums ? h->C_sums : h->C;
   cudaError_t e = cudaErrorInvalidValue;
-  timed(h, kind, [&] { e = launch_move_side(h->N, C, MODE, a, nslot, K, h->stream); }, nslot);
+  timed(h, kind, [&] { e = launch_move_side(h->N, h->C, MODE, a, nslot, K, h->stream); }, nslot);
   return e;
 }
 

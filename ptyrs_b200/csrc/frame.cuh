@@ -298,6 +298,18 @@ __global__ void __launch_bounds__(PlaneShape<N, C>::T,
     }
   };
 
+  // What the cluster reads after the first row transforms, fetched into L2 now (256² x 2 gradient
+  // 1.883 -> 1.854 us per frame, carry 2.214 -> 2.192, rPIE 128² x 2 0.545 -> 0.518; at 64² the
+  // addresses cost more than the loads' latency).
+  if (!from_field && N > 64) {
+    L::prefetch_columns(a.iobs + (size_t)f * plane + r * H);
+    for (int m = 1; m < K; ++m) {
+      const size_t row = ((size_t)slot * K + m) * plane + (size_t)ny * N;
+      if (a.probe_stride) ln.prefetch_row(a.probe + row);
+      if (MODE == kCarry && a.c_psi != 0.f) ln.prefetch_row(a.carry + row);
+      if (MODE == kCarry && a.c_it != 0.f) ln.prefetch_row(a.iter + row);
+    }
+  }
   float2 v[E];
   if (!from_field) {
     // Exit waves ψ = P·O·q of the rows, mode by mode; (P·O)·q as P·(O·q): the reference's

@@ -173,6 +173,21 @@ struct Lines {
     }
   }
 
+  // Fetches this CTA's part of a global plane [N][N] into L2 ahead of its use: the row of this
+  // row-mapped thread (`row0` its first element), or the CTA's columns r·H .. of every ky
+  // (`col0` the first of them), for elements of B bytes.
+  template <typename V>
+  PTYB_D void prefetch_row(const V* row0) const {
+    constexpr int kLines = N * (int)sizeof(V) / 128;
+    for (int l = rt; l < kLines; l += N2) prefetch(reinterpret_cast<const char*>(row0) + l * 128);
+  }
+  template <typename V>
+  static PTYB_D void prefetch_columns(const V* col0) {
+    constexpr int kSpan = H * (int)sizeof(V), kLines = (kSpan + 127) / 128;
+    for (int i = threadIdx.x; i < N * kLines; i += T)
+      prefetch(reinterpret_cast<const char*>(col0 + (size_t)(i / kLines) * N) + (i % kLines) * 128);
+  }
+
   // Every CTA's lines visible to the cluster.
   static PTYB_D void publish() {
     if (C > 1) {
@@ -232,6 +247,9 @@ struct Lines {
   }
 
  private:
+  static PTYB_D void prefetch(const void* a) {
+    asm volatile("prefetch.global.L2 [%0];" ::"l"(a));
+  }
   PTYB_D void exchange(float2 (&v)[N1], int m) const {
     stash(v, m);
     __syncthreads();

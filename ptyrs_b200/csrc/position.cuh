@@ -59,7 +59,8 @@ __host__ __device__ constexpr size_t move_smem_bytes(int K) {
 // (or a spectrum read in the columns), the phase in the columns, inverse to natural rows. As the
 // frame kernel, bound by latency (its exchanges and cluster barriers); per frame on one B200 at
 // 256² x 2 modes: moves from the spectrum 1.42 -> 0.93 us, probe gradient spectra 1.57 -> 1.03,
-// position sums 3.21 -> 2.21 (four inverse transforms), one plane's spectrum 27 -> 16 us a call.
+// position sums 3.21 -> 2.21 (four inverse transforms; 2.15 -> 2.0 on the frame kernels' clusters
+// of 16 instead of 8), one plane's spectrum 27 -> 16 us a call.
 template <int N, int C, int MODE>
 __global__ void __launch_bounds__(PlaneShape<N, C>::T,
                                   plane_min_blocks<N, C>(MODE != kDerivSums &&
