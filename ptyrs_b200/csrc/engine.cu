@@ -552,7 +552,8 @@ void download_c64(ptyb_handle* h, const float2* src, double* dst, size_t n, cons
   std::lock_guard<std::mutex> lock(g_stage_mutex);
   float2* st = staging(h, n);
   check(h, copy_sync(h, st, src, n * sizeof(float2), cudaMemcpyDeviceToHost), what);
-  parallel_range(n, [&](size_t b, size_t e) {
+  // the caller's fresh array is first touched here: 777² values took 2.1 ms on one thread
+  parallel_range(n, size_t(1) << 16, 16, [&](size_t b, size_t e) {
     for (size_t i = b; i < e; ++i) {
       dst[2 * i] = st[i].x;
       dst[2 * i + 1] = st[i].y;
@@ -564,7 +565,9 @@ void download_c64(ptyb_handle* h, const float2* src, double* dst, size_t n, cons
 void upload_c64(ptyb_handle* h, const double* src, float2* dst, size_t n, const char* what) {
   std::lock_guard<std::mutex> lock(g_stage_mutex);
   float2* st = staging(h, n);
-  parallel_range(n, [&](size_t b, size_t e) {
+  // (both arrays are in memory already: below 2^20 values the threads cost what they save)
+  const size_t each = n < (size_t(1) << 20) ? n + 1 : n / 8;
+  parallel_range(n, each, 8, [&](size_t b, size_t e) {
     for (size_t i = b; i < e; ++i) st[i] = make_float2((float)src[2 * i], (float)src[2 * i + 1]);
   });
   check(h, copy_sync(h, dst, st, n * sizeof(float2), cudaMemcpyHostToDevice), what);

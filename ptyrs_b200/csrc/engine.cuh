@@ -337,13 +337,11 @@ bool llk_due(int calc_llk, int ic, int ncycle);
 void upload_orders(ptyb_handle* h, int nepoch, int size, uint64_t seed, int64_t epoch0,
                    std::vector<std::vector<int32_t>>* sizes, std::vector<int32_t>* last);
 
-// Runs fn(begin, end) over [0, n) on up to sixteen host threads, one for every 2^16 values: the
-// conversion of a 777² object and the first touch of its 9.7 MB took 2.1 ms on one thread, where
-// only arrays above 2^20 values were cut.
+// Runs fn(begin, end) over [0, n) on up to `most` host threads, each of at least `each` values.
 template <class F>
-void parallel_range(size_t n, F&& fn) {
-  const size_t nt = std::min<size_t>({16, std::max(1u, std::thread::hardware_concurrency()),
-                                      n >> 16});
+void parallel_range(size_t n, size_t each, size_t most, F&& fn) {
+  const size_t nt = std::min<size_t>({most, std::max(1u, std::thread::hardware_concurrency()),
+                                      n / each});
   if (nt <= 1) {
     fn(size_t(0), n);
     return;
