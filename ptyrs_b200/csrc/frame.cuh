@@ -99,13 +99,6 @@ struct FrameShape {
   static constexpr int E = H * N / T;       // = 16
 };
 
-// Resident CTAs per SM the per-frame kernels are compiled for: two at 384 threads or fewer
-// (a cap of 128 registers at 256 threads, 113 at the 288 of sides 96 and 192), one above.
-template <int N, int C>
-__host__ __device__ constexpr int frame_min_blocks() {
-  return FrameShape<N, C>::T <= 384 ? 2 : 1;
-}
-
 template <int N, int C>
 __host__ __device__ constexpr size_t frame_smem_bytes(int K) {
   return (size_t)K * FrameShape<N, C>::H * FrameShape<N, C>::L * sizeof(float2) +
