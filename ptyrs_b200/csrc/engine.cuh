@@ -20,6 +20,7 @@
 
 #include "../../include/ptyb200.h"
 #include "gather.cuh"
+#include "host_threads.h"
 #include "launch.cuh"
 #include "lsqml.cuh"
 #include "ml.cuh"
@@ -336,24 +337,6 @@ void record(ptyb_handle* h, int algorithm, const ptyb_llk& l);
 bool llk_due(int calc_llk, int ic, int ncycle);
 void upload_orders(ptyb_handle* h, int nepoch, int size, uint64_t seed, int64_t epoch0,
                    std::vector<std::vector<int32_t>>* sizes, std::vector<int32_t>* last);
-
-// Runs fn(begin, end) over [0, n) on up to `most` host threads, each of at least `each` values.
-template <class F>
-void parallel_range(size_t n, size_t each, size_t most, F&& fn) {
-  const size_t nt = std::min<size_t>({most, std::max(1u, std::thread::hardware_concurrency()),
-                                      n / each});
-  if (nt <= 1) {
-    fn(size_t(0), n);
-    return;
-  }
-  std::vector<std::thread> ts;
-  const size_t chunk = (n + nt - 1) / nt;
-  for (size_t t = 0; t < nt; ++t) {
-    const size_t b = t * chunk, e = std::min(n, b + chunk);
-    if (b < e) ts.emplace_back([&fn, b, e] { fn(b, e); });
-  }
-  for (auto& t : ts) t.join();
-}
 
 void download_c64(ptyb_handle* h, const float2* src, double* dst, size_t n, const char* what);
 void upload_c64(ptyb_handle* h, const double* src, float2* dst, size_t n, const char* what);
