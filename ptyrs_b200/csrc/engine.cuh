@@ -34,9 +34,11 @@
 constexpr int kMaxSlices = 16;
 // Room for the kernel kinds of the per-kernel timing (the Kind enum below fits it).
 constexpr int kMaxKinds = 48;
-constexpr int kScalars = 8 + kMaxSlices + 2;
-// The maxima of the AP / DM / RAAR blends' object and probe norms.
-constexpr int kScalObjNorm = 8 + kMaxSlices, kScalProbeNorm = kScalObjNorm + 1;
+constexpr int kScalars = 8 + kMaxSlices + 4;
+// The maxima of the AP / DM / RAAR blends' object and probe norms; the largest overlap of an rPIE
+// batch and of the next, in turn.
+constexpr int kScalObjNorm = 8 + kMaxSlices, kScalProbeNorm = kScalObjNorm + 1,
+              kScalOverlap = kScalProbeNorm + 1;
 
 namespace ptyb::eng {
 
@@ -161,11 +163,10 @@ struct ptyb_handle {
   double* pcg_norms = nullptr;    // [P][K]
   double* pcg_modes = nullptr;    // [K][2]
   double* partials = nullptr;    // [kPartialBlocks][2]
-  // rPIE: a batch's object sums and overlaps per mode [K][nyo][nxo], the largest overlap of this
-  // batch and the next.
+  // rPIE: a batch's object sums and overlaps per mode [K][nyo][nxo], where no array that the
+  // handle holds anyway has the room (rpie.cu, batch_sums).
   float2* rpie_num = nullptr;
   float* rpie_den = nullptr;
-  float* rpie_max = nullptr;
   // Phase-ramp removal: the probe's row transforms [K][N][N], the columns' sums [K·N][3] and
   // the centroid's offset (dy, dx) behind them.
   double2* ramp_rows = nullptr;

@@ -8,12 +8,37 @@ using namespace ptyb;
 namespace ptyb::eng {
 namespace {
 
+// The arrays that take a batch's object sums and overlaps per mode, [K][nyo][nxo].
+struct BatchSums {
+  float2* num;
+  float* den;
+};
+
+// For one mode they are LSQML's direction and preconditioner, which no call leaves a value in for
+// another; for more, the part of the frames' planes (h->field) that batches of `batch` frames
+// leave alone: all of it, or past the batch's own planes under the position model. Only where the
+// object is larger than that (12·K bytes a pixel) do they get arrays of their own, made once.
+BatchSums batch_sums(ptyb_handle* h, int batch) {
+  if (h->K == 1) return {h->d_obj, h->pre};
+  const size_t n = (size_t)h->K * h->nyo * h->nxo, planes = (size_t)h->K * h->N * h->N;
+  const size_t used = h->have_offsets ? batch * planes : 0;
+  if (8 * (h->slots * planes - used) >= 12 * n) {
+    float2* num = h->field + used;
+    return {num, reinterpret_cast<float*>(num + n)};
+  }
+  if (!h->rpie_num) {
+    h->rpie_num = alloc<float2>(h, n);
+    h->rpie_den = alloc<float>(h, n);
+  }
+  return {h->rpie_num, h->rpie_den};
+}
+
 // One rPIE batch (engine/ptycho.rs:904-1085; GPU launch sequence engine/gpu/rpie.rs:239-345):
 // the frame pass, the object and probe sums from the batch-start arrays, the position model's
 // passes, then both updates. `pmax` and `pmax_next` take the largest overlap of this batch and
-// of the next in turn (h->rpie_max), each cleared by the updates of the batch before.
+// of the next in turn, each cleared by the updates of the batch before.
 void rpie_batch(ptyb_handle* h, const ptyb_rpie_params& p, const int* frames, int nslot,
-                float* pmax, float* pmax_next) {
+                const BatchSums& sums, float* pmax, float* pmax_next) {
   FrameArgs a = frame_args(h, frames);
   GatherArgs g = gather_args(h, frames, nslot);
   const int pstride = h->K * h->N * h->N;
@@ -38,8 +63,8 @@ void rpie_batch(ptyb_handle* h, const ptyb_rpie_params& p, const int* frames, in
   const int chunk = sum_probe ? probe_chunk(h, nslot, &nchunk) : 0;
   const int tiles = p.update_object ? ntiles(h) : 0, pblocks = nchunk * (h->N * h->N / kTileThreads);
   if (tiles + pblocks > 0) {
-    g.out = h->rpie_num;
-    g.pre = h->rpie_den;
+    g.out = sums.num;
+    g.pre = sums.den;
     g.pmax = pmax;
     ProbeArgs pa = {};
     pa.object = h->object;
@@ -82,8 +107,8 @@ void rpie_batch(ptyb_handle* h, const ptyb_rpie_params& p, const int* frames, in
   // O and P += step/nbatch · Σ (frames in order)
   RpieApplyArgs u = {};
   u.object = h->object;
-  u.num = h->rpie_num;
-  u.den = h->rpie_den;
+  u.num = sums.num;
+  u.den = sums.den;
   u.pmax = pmax;
   u.pmax_next = pmax_next;
   u.probe = h->probe;
@@ -138,20 +163,16 @@ int ptyb_rpie(ptyb_handle* h, const ptyb_rpie_params* p, int32_t nepoch) {
     ensure_slots(h, std::max(bs, std::min(h->P, h->stack)));
     std::vector<std::vector<int32_t>> sizes;
     upload_orders(h, nepoch, p->batch_size, p->seed, h->cycle, &sizes, nullptr);
-    if (!h->rpie_num) {
-      const size_t no = (size_t)h->nyo * h->nxo;
-      h->rpie_num = alloc<float2>(h, h->K * no);
-      h->rpie_den = alloc<float>(h, h->K * no);
-      h->rpie_max = alloc<float>(h, 2);
-    }
+    const BatchSums sums = batch_sums(h, bs);
+    float* overlap = h->scal + kScalOverlap;
     begin_call(h);
-    check(h, cudaMemsetAsync(h->rpie_max, 0, 2 * sizeof(float), h->stream), "memset");
+    check(h, cudaMemsetAsync(overlap, 0, 2 * sizeof(float), h->stream), "memset");
     int64_t batch = 0;
     for (int ic = 0; ic < nepoch; ++ic) {
       const int* order = h->order_all + (size_t)ic * h->P;
       int off = 0;
       for (int n : sizes[ic]) {
-        rpie_batch(h, *p, order + off, n, h->rpie_max + batch % 2, h->rpie_max + (batch + 1) % 2);
+        rpie_batch(h, *p, order + off, n, sums, overlap + batch % 2, overlap + (batch + 1) % 2);
         off += n;
         ++batch;
       }
