@@ -622,21 +622,26 @@ unsigned blocks_for(size_t n) { return (unsigned)((n + 255) / 256); }
 void zero_phase_ramp(ptyb_handle* h) {
   const int N = h->N;
   const size_t plane = (size_t)N * N;
-  if (!h->ramp_rows) {
-    h->ramp_rows = alloc<double2>(h, (size_t)h->K * plane);
-    h->ramp_sums = alloc<double>(h, (size_t)h->K * N * 3 + 2);
+  // After a call's last cycle the frames' planes and LSQML's probe direction hold nothing: the
+  // probe's row transforms [K][N][N] go to the first, the columns' sums [K·N][3] and the
+  // centroid's offset (dy, dx) behind them to the second.
+  auto* rows = reinterpret_cast<double2*>(h->field);
+  if (h->slots * std::max(h->K, 2) < 2 * h->K) {
+    if (!h->ramp_rows) h->ramp_rows = alloc<double2>(h, (size_t)h->K * plane);
+    rows = h->ramp_rows;
   }
-  double* shift = h->ramp_sums + (size_t)h->K * N * 3;
+  auto* sums = reinterpret_cast<double*>(h->d_probe);
+  double* shift = sums + (size_t)h->K * N * 3;
   const dim3 lines(N, h->K);
   const size_t smem = 2 * (size_t)N * sizeof(double2);
-  timed(h, kKMisc, [&] { ramp_rows_kernel<<<lines, N, smem, h->stream>>>(h->probe, N, h->ramp_rows); });
+  timed(h, kKMisc, [&] { ramp_rows_kernel<<<lines, N, smem, h->stream>>>(h->probe, N, rows); });
   launched(h, "probe far field rows");
   timed(h, kKMisc, [&] {
-    ramp_columns_kernel<<<lines, N, smem, h->stream>>>(h->ramp_rows, N, h->ramp_sums);
+    ramp_columns_kernel<<<lines, N, smem, h->stream>>>(rows, N, sums);
   });
   launched(h, "probe far field columns");
   timed(h, kKMisc, [&] {
-    ramp_centroid_kernel<<<1, 32, 0, h->stream>>>(h->ramp_sums, h->K * N, N, shift);
+    ramp_centroid_kernel<<<1, 32, 0, h->stream>>>(sums, h->K * N, N, shift);
   });
   launched(h, "probe far field centroid");
   const size_t np = (size_t)h->K * plane, no = (size_t)h->nobj * h->nyo * h->nxo;

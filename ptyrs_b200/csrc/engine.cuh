@@ -167,10 +167,9 @@ struct ptyb_handle {
   // handle holds anyway has the room (rpie.cu, batch_sums).
   float2* rpie_num = nullptr;
   float* rpie_den = nullptr;
-  // Phase-ramp removal: the probe's row transforms [K][N][N], the columns' sums [K·N][3] and
-  // the centroid's offset (dy, dx) behind them.
+  // Phase-ramp removal: the probe's row transforms [K][N][N], where h->field has no room for them
+  // (launches of one frame).
   double2* ramp_rows = nullptr;
-  double* ramp_sums = nullptr;
   std::vector<ptyb::eng::Buf> bufs;
   // Per-kernel device timing (CUDA events on the engine's stream), when enabled.
   bool timing = false;

@@ -7,7 +7,8 @@ import pytest
 
 from oracle.ptycho import zero_phase_ramp
 from ptyrs_b200 import GpuPtycho, Scan, sim
-from scenarios import rel_l2
+from scenarios import far_field, rel_l2
+from test_zz_no_alloc import _driver, _pool_used
 
 pytestmark = pytest.mark.gpu
 
@@ -30,3 +31,28 @@ def test_ramp_of_a_call_without_cycles(n, modes):
         g.ap(0, zero_phase_ramp=True)
         assert rel_l2(g.probe(), want_probe) < 1e-6
         assert rel_l2(g.object(), want_obj) < 1e-6
+
+
+@pytest.mark.parametrize("modes,stack,own", [(1, 1, False), (2, 2, False), (3, 2, False),
+                                             (3, 1, True)])
+def test_ramp_lies_in_memory_held_anyway(modes, stack, own):
+    """The removal takes no device memory of its own, but for several modes with launches of one
+    frame (16·K·N² bytes, once)."""
+    cu = _driver()
+    s = far_field(64, modes, 4, 128, seed=modes)
+    scan = Scan(s["counts"], s["y"], s["x"], sim.WAVELENGTH, sim.DISTANCE, sim.DETECTOR_PIXEL)
+    obj, probe = s["truth"], s["probe"] * (1 + 0.1j)
+    with GpuPtycho(scan, obj, probe, stack_size=stack) as g:
+        g.ap(0, zero_phase_ramp=False)
+        used = _pool_used(cu)
+        g.ap(0, zero_phase_ramp=True)
+        want_obj, want_probe = zero_phase_ramp(obj.astype(np.complex64).astype(complex),
+                                               probe.astype(np.complex64).astype(complex))
+        assert rel_l2(g.probe(), want_probe) < 1e-6
+        assert rel_l2(g.object(), want_obj) < 1e-6
+        g.ap(0, zero_phase_ramp=True)
+        more = _pool_used(cu) - used
+    if own:
+        assert 16 * modes * 64 ** 2 <= more < 17 * modes * 64 ** 2
+    else:
+        assert more == 0
