@@ -233,7 +233,8 @@ def algorithmic_bytes(kind, s, wl):
         "probe_partial": 8 * K * n2 + 8 * n2,
         "lsqml_dots": 8 * K * n2 + 16 * n2,
         "object_lsqml": 8 * K * n2,
-        "object_rpie": 8 * K * n2,
+        # rPIE's object and probe sums in one launch: the update planes and the object window
+        "rpie_sums": 8 * K * n2 + 8 * n2,
         "object_ml": 8 * K * n2 + moved,
         # AP / DM / RAAR: object window, counts, the carried waves read and written (RAAR also
         # its iterate)

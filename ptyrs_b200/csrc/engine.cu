@@ -193,7 +193,7 @@ void launched(ptyb_handle* h, const char* what) {
 
 const char* const kKindNames[kNumKinds] = {
     "frame_rpie", "frame_lsqml", "frame_ml_grad", "frame_llk", "frame_store",
-    "frame_from_store", "object_rpie", "object_lsqml", "object_ml",
+    "frame_from_store", "rpie_sums", "rpie_updates", "object_lsqml", "object_ml",
     "illumination", "probe_partial", "probe_finalize", "lsqml_afar", "lsqml_dots",
     "lsqml_solve", "axpy", "max", "counts", "misc", "ml_gamma", "array_sums", "move",
     "position_sums", "slice_forward", "slice_backward", "slice_llk", "frame_project", "spectrum",

@@ -237,7 +237,7 @@ constexpr int kPartialBlocks = 296;
 // Kernel kinds for the per-kernel timing (ptyb_kernel_name).
 enum Kind : int {
   kKFrameRpie = 0, kKFrameLsqml, kKFrameMl, kKFrameLlk, kKFrameStore, kKFrameFromStore,
-  kKObjRpie, kKObjLsqml, kKObjMl, kKIllum, kKProbePartial, kKProbeFinal,
+  kKRpieSums, kKRpieUpdates, kKObjLsqml, kKObjMl, kKIllum, kKProbePartial, kKProbeFinal,
   kKAfar, kKDots, kKSolve, kKAxpy, kKMax, kKCounts, kKMisc, kKGamma, kKArraySums, kKMove,
   kKPositionSums, kKSliceForward, kKSliceBackward, kKSliceLlk, kKFrameProject, kKSpectrum,
   kKDerivSums, kKBackSpectrum, kKSliceGrad, kKFrameCarry, kKObjBlend, kKOprStep, kKBhHessian,

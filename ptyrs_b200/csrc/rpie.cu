@@ -80,7 +80,7 @@ void rpie_batch(ptyb_handle* h, const ptyb_rpie_params& p, const int* frames, in
     pa.nxo = h->nxo;
     pa.K = h->K;
     pa.N = h->N;
-    timed(h, kKObjRpie, [&] { launch_rpie_sums(g, pa, tiles, tiles + pblocks, h->stream); }, nslot);
+    timed(h, kKRpieSums, [&] { launch_rpie_sums(g, pa, tiles, tiles + pblocks, h->stream); }, nslot);
     launched(h, "rpie sums");
   }
   if (refine) {
@@ -122,7 +122,7 @@ void rpie_batch(ptyb_handle* h, const ptyb_rpie_params& p, const int* frames, in
   u.step = (float)p.obj_step;
   u.coef = (float)(p.probe_step / nslot);
   if (u.oblocks + u.count > 0) {
-    timed(h, kKProbeFinal, [&] {
+    timed(h, kKRpieUpdates, [&] {
       rpie_apply_kernel<<<u.oblocks + blocks_for(u.count), 256, 0, h->stream>>>(u);
     });
     launched(h, "rpie updates");

@@ -1,7 +1,9 @@
-"""Host logic of the bench's time-to-target leg (no GPU): LLK records to per-iteration traces
-and the reference's two-target rule."""
+"""Host logic of the bench (no GPU): its kernels' byte counts, and of its time-to-target leg the
+LLK records to per-iteration traces and the reference's two-target rule."""
 import os
 import sys
+
+import numpy as np
 
 sys.path.insert(0, os.path.dirname(os.path.dirname(os.path.abspath(__file__))))
 
@@ -38,3 +40,18 @@ def test_a_diverged_run_sets_no_target():
     (t1, i1), (t2, i2) = targets
     assert t1 == 1.01 * 1.0 and i1 == {"rpie": None, "lsqml": None, "ml": 3}
     assert t2 == 1.01 * 1.1 and i2 == {"rpie": None, "lsqml": 3, "ml": 3}
+
+
+def test_rpie_bytes_are_those_of_its_launches():
+    """rPIE's sums (object and probe in one launch) have their bytes under the name that the
+    library times them by; the updates run over object and probe pixels, not frames."""
+    from ptyrs_b200 import _lib, build
+    build.build()
+    lib = _lib.load()
+    names = {lib.ptyb_kernel_name(i).decode() for i in range(lib.ptyb_kernel_kinds())}
+    assert {"frame_rpie", "rpie_sums", "rpie_updates"} <= names and "object_rpie" not in names
+    s = dict(n=64, probe=np.ones((2, 64, 64)), object=np.ones((1, 256, 256)))
+    wl = dict(algorithm="rpie")
+    assert bench.algorithmic_bytes("rpie_sums", s, wl) == (2 * 8 + 8) * 64 ** 2
+    assert bench.algorithmic_bytes("rpie_updates", s, wl) is None
+    assert bench.algorithmic_bytes("object_rpie", s, wl) is None
