@@ -93,7 +93,6 @@ void bh_grads(ptyb_handle* h, const int* frames, int n) {
     pa.upd = gfield;
     pa.frames = fr;
     pa.corners = h->corners;
-    pa.omax = h->omax;
     pa.partial = h->partial;
     pa.nslot = m;
     pa.chunk = chunk;

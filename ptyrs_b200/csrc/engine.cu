@@ -337,7 +337,6 @@ GatherArgs gather_args(ptyb_handle* h, const int* frames, int nslot) {
   g.upd = h->upd;
   g.frames = frames;
   g.corners = h->corners;
-  g.pmax = h->scal + 0;
   g.pre = h->pre;
   g.pre_max = h->scal + 1;
   g.out = h->d_obj;
@@ -391,12 +390,10 @@ int probe_chunk(ptyb_handle* h, int nslot, int* nchunk) {
   return chunk;
 }
 
-// Σ_frames (w·upd) into the probe (mode 0: P += coef·Σ with the rPIE weight; 1: d_probe =
-// coef·Σ conj(q·O)·upd).
-// Probe direction Σ w·upd over the batch; `quad` and `upd` default to the exit phase and the
-// frame kernel's update planes.
-void probe_pass(ptyb_handle* h, const int* frames, int nslot, int mode, float alpha, float coef,
-                const float2* quad, const float2* upd) {
+// The batch's probe direction d_probe = coef·Σ_frames conj(q·O)·upd; `quad` and `upd` default to
+// the exit phase and the frame kernel's update planes.
+void probe_pass(ptyb_handle* h, const int* frames, int nslot, float coef, const float2* quad,
+                const float2* upd) {
   int nchunk = 0;
   const int chunk = probe_chunk(h, nslot, &nchunk);
   ProbeArgs p = {};
@@ -405,21 +402,19 @@ void probe_pass(ptyb_handle* h, const int* frames, int nslot, int mode, float al
   p.upd = upd ? upd : h->upd;
   p.frames = frames;
   p.corners = h->corners;
-  p.omax = h->omax;
   p.partial = h->partial;
-  p.alpha = alpha;
   p.nslot = nslot;
   p.chunk = chunk;
   p.nxo = h->nxo;
   p.K = h->K;
   p.N = h->N;
-  p.mode = mode == 0 ? 0 : 1;
+  p.mode = 1;
   timed(h, kKProbePartial, [&] { launch_probe_partial(p, nchunk, h->stream); }, nslot);
   launched(h, "probe_partial");
   const int count = h->K * h->N * h->N;
   timed(h, kKProbeFinal, [&] {
-  probe_finalize_kernel<<<(count + 255) / 256, 256, 0, h->stream>>>(
-      h->partial, nchunk, count, h->probe, h->d_probe, nullptr, coef, mode);
+    probe_finalize_kernel<<<(count + 255) / 256, 256, 0, h->stream>>>(
+        h->partial, nchunk, count, h->probe, h->d_probe, nullptr, coef, 1);
   });
   launched(h, "probe_finalize");
 }

@@ -85,7 +85,7 @@ struct ptyb_handle {
   float* afar2 = nullptr;     // [slots]
   float2* partial = nullptr;  // [nchunk][K][N][N]
   int max_chunks = 0;
-  float* scal = nullptr;      // [8]: pmax, pre max, object step, probe step
+  float* scal = nullptr;      // [kScalars]: 1 pre max, 2 object, 3 probe and 4.. slice steps
   float* pre = nullptr;       // [nyo][nxo]
   float2* d_obj = nullptr;    // [nyo][nxo]
   float2* d_probe = nullptr;  // [K][N][N]
@@ -329,7 +329,7 @@ GatherArgs gather_args(ptyb_handle* h, const int* frames, int nslot);
 int ntiles(ptyb_handle* h);
 void ensure_slots(ptyb_handle* h, int n);
 int probe_chunk(ptyb_handle* h, int nslot, int* nchunk);
-void probe_pass(ptyb_handle* h, const int* frames, int nslot, int mode, float alpha, float coef,
+void probe_pass(ptyb_handle* h, const int* frames, int nslot, float coef,
                 const float2* quad = nullptr, const float2* upd = nullptr);
 ptyb_llk llk_pass(ptyb_handle* h, const float2* waves = nullptr);
 ptyb_llk llk_of_frames(ptyb_handle* h);

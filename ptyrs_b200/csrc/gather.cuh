@@ -287,29 +287,25 @@ struct ProbeArgs {
   const int2* corners;
   const float* omax;      // rPIE [slot]
   float2* partial;        // [nchunk][K][N][N]
-  float* partial_den;     // mode 2: [nchunk][N][N] Σ_slots |O|² over the window
-  float alpha;
-  // mode 0 rPIE weight, 1 plain conj(q·O), 2 also Σ|O|², 3 Σ|O|² alone
+  float* partial_den;     // modes 2 and 3: [nchunk][N][N] Σ_slots |O|² over the window
+  float alpha;            // rPIE
+  // probe_partial_kernel: 1 Σ conj(q·O)·upd, 2 also Σ|O|², 3 Σ|O|² alone
   int nslot, chunk, nxo, K, N, mode;
 };
 
 constexpr int kMaxProbeChunk = 256;
 
 // Chunk `blockIdx.y` of slots (at most kMaxProbeChunk), 512 probe pixels per CTA of 256 threads:
-// Σ_slots w·upd in slot order for a's K modes. Two neighbouring pixels a thread, the update
+// Σ_slots conj(q·O)·upd in slot order for a's K modes. Two neighbouring pixels a thread, the update
 // planes and the phase read 16 bytes at a time: bound by the latency of those loads (84 % of the
 // stalls with one pixel a thread).
 template <int K>
 static __global__ void __launch_bounds__(256) probe_partial_kernel(ProbeArgs a) {
   __shared__ int2 cs[kMaxProbeChunk];
-  __shared__ float om[kMaxProbeChunk];
   const int N = a.N;
   const size_t plane = (size_t)N * N;
   const int s0 = blockIdx.y * a.chunk, s1 = min(a.nslot, s0 + a.chunk);
-  for (int i = threadIdx.x; i < s1 - s0; i += 256) {
-    cs[i] = a.corners[a.frames[s0 + i]];
-    om[i] = a.mode == 0 ? a.omax[s0 + i] : 0.f;
-  }
+  for (int i = threadIdx.x; i < s1 - s0; i += 256) cs[i] = a.corners[a.frames[s0 + i]];
   __syncthreads();
   const int pix = 2 * (blockIdx.x * 256 + threadIdx.x);
   if (pix >= N * N) return;
@@ -337,11 +333,7 @@ static __global__ void __launch_bounds__(256) probe_partial_kernel(ProbeArgs a) 
     if (a.mode == 3) continue;
     float2 w[2];  // conjugated in the products below
 #pragma unroll
-    for (int j = 0; j < 2; ++j) {
-      w[j] = cmul_rn(o[j], q[j]);
-      if (a.mode == 0)
-        w[j] = cscale(w[j], 1.f / ((1.f - a.alpha) * cnorm2(o[j]) + a.alpha * om[s - s0]));
-    }
+    for (int j = 0; j < 2; ++j) w[j] = cmul_rn(o[j], q[j]);
 #pragma unroll
     for (int m = 0; m < K; ++m) {
       const float4 u =
@@ -364,8 +356,8 @@ static __global__ void __launch_bounds__(256) probe_partial_kernel(ProbeArgs a) 
 }
 
 // rPIE's object sums (the first `ntiles` blocks, one object tile each) and probe sums (the rest:
-// kTileThreads pixels of one chunk of slots, one a thread, mode 0's weight) of a batch in one
-// launch. Both read the batch-start object and probe, and at 64² neither fills the GPU for more
+// kTileThreads pixels of one chunk of slots, one a thread, Σ w·upd with the weight
+// w = conj(q·O)/((1−α)|O|² + α·max|O|²)) of a batch in one launch. Both read the batch-start object and probe, and at 64² neither fills the GPU for more
 // than the latency of a few views. With the maximum of the overlaps taken here and the updates in
 // rpie_apply_kernel a batch is three launches instead of five: frame pass, sums, updates (46 ->
 // 28 us for 100 frames of 64²).
@@ -573,8 +565,7 @@ static __global__ void __launch_bounds__(256) probe_norm_kernel(const float* par
   }
 }
 
-// Σ over chunks in order; mode 0: P += coef·Σ; 1: out = coef·Σ; 2: out += Σ compensated;
-// 3: the blend P = (Σ + reg·P) / max(norm + reg, 1e-12) with reg = coef·max norm
+// Σ over chunks in order; mode 1: out = coef·Σ; 2: out += Σ compensated; 3: the blend P = (Σ + reg·P) / max(norm + reg, 1e-12) with reg = coef·max norm
 // (engine/ops.rs:371-381), `norm` one plane shared by the modes.
 static __global__ void probe_finalize_kernel(const float2* partial, int nchunk, int count,
                                       float2* probe, float2* out, float2* comp, float coef,
@@ -583,9 +574,7 @@ static __global__ void probe_finalize_kernel(const float2* partial, int nchunk, 
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= count) return;
   const float2 v = plane_sum(partial, nchunk, count, i);
-  if (mode == 0) {
-    probe[i] = cadd(probe[i], cscale(v, coef));
-  } else if (mode == 3) {
+  if (mode == 3) {
     const float reg = coef * (*norm_max);
     probe[i] = cscale(cadd(v, cscale(probe[i], reg)), 1.f / fmaxf(norm[i % plane] + reg, 1e-12f));
   } else if (mode == 1) {

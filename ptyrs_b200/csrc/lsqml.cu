@@ -135,7 +135,7 @@ void lsqml_batch_slices(ptyb_handle* h, const ptyb_lsqml_params& p, const int* f
   if (own)
     dirs = probe_directions(h, frames, nslot, h->ones, h->chi_slices);
   else
-    probe_pass(h, frames, nslot, 1, 0.f, 1.0f / nslot, h->ones, h->chi_slices);
+    probe_pass(h, frames, nslot, 1.0f / nslot, h->ones, h->chi_slices);
   const double lambda0 = 1.2e-7 * ((double)h->N * h->N) / ((double)h->N * h->N);
   timed(h, kKDots, [&] {
     lsqml_dots_kernel<<<nslot * kDotParts, 512, 0, h->stream>>>(
@@ -351,7 +351,7 @@ void lsqml_batch(ptyb_handle* h, const ptyb_lsqml_params& p, const int* frames, 
   if (own)
     dirs = probe_directions(h, frames, nslot, h->quad, h->upd);
   else
-    probe_pass(h, frames, nslot, 1, 0.f, 1.0f / nslot);
+    probe_pass(h, frames, nslot, 1.0f / nslot);
   const double lambda0 = 1.2e-7 * ((double)h->N * h->N) / ((double)h->N * h->N);
   const float2* fprobe = own ? own : h->probe;
   const int fstride = own ? pstride : 0;

@@ -68,7 +68,6 @@ void slice_gradients(ptyb_handle* h, bool uo, bool up, const int* frames_in, int
       pa.upd = h->chi_slices;
       pa.frames = frames;
       pa.corners = h->corners;
-      pa.omax = h->omax;
       pa.partial = h->partial;
       pa.nslot = n;
       pa.chunk = chunk;
@@ -174,7 +173,6 @@ void ml_gradients(ptyb_handle* h, bool uo, bool up, bool refine, bool pos_grad =
       pa.upd = gfield;
       pa.frames = frames;
       pa.corners = h->corners;
-      pa.omax = h->omax;
       pa.partial = h->partial;
       pa.nslot = n;
       pa.chunk = chunk;
