@@ -294,8 +294,10 @@ struct ProbeArgs {
 };
 
 constexpr int kMaxProbeChunk = 256;
+constexpr int kProbePixels = 512;  // probe pixels per CTA of the probe sums, rPIE's too
+static_assert(kProbePixels == kTileThreads, "rpie_sums_kernel takes a probe pixel a thread");
 
-// Chunk `blockIdx.y` of slots (at most kMaxProbeChunk), 512 probe pixels per CTA of 256 threads:
+// Chunk `blockIdx.y` of slots (at most kMaxProbeChunk), kProbePixels pixels per CTA of 256 threads:
 // Σ_slots conj(q·O)·upd in slot order for a's K modes. Two neighbouring pixels a thread, the update
 // planes and the phase read 16 bytes at a time: bound by the latency of those loads (84 % of the
 // stalls with one pixel a thread).
@@ -356,11 +358,11 @@ static __global__ void __launch_bounds__(256) probe_partial_kernel(ProbeArgs a) 
 }
 
 // rPIE's object sums (the first `ntiles` blocks, one object tile each) and probe sums (the rest:
-// kTileThreads pixels of one chunk of slots, one a thread, Σ w·upd with the weight
-// w = conj(q·O)/((1−α)|O|² + α·max|O|²)) of a batch in one launch. Both read the batch-start object and probe, and at 64² neither fills the GPU for more
-// than the latency of a few views. With the maximum of the overlaps taken here and the updates in
-// rpie_apply_kernel a batch is three launches instead of five: frame pass, sums, updates (46 ->
-// 28 us for 100 frames of 64²).
+// kProbePixels pixels of one chunk of slots, one a thread, Σ w·upd with the weight w =
+// conj(q·O)/((1−α)|O|² + α·max|O|²)) of a batch in one launch. Both read the batch-start object and
+// probe, and at 64² neither fills the GPU for more than the latency of a few views. With the
+// maximum of the overlaps taken here and the updates in rpie_apply_kernel a batch is three launches
+// instead of five: frame pass, sums, updates (46 -> 28 us for 100 frames of 64²).
 template <int K>
 static __global__ void __launch_bounds__(kTileThreads, tile_min_blocks<kGatherRpie, K>())
     rpie_sums_kernel(GatherArgs g, ProbeArgs a, int ntiles) {
@@ -370,7 +372,7 @@ static __global__ void __launch_bounds__(kTileThreads, tile_min_blocks<kGatherRp
   }
   __shared__ int2 cs[kMaxProbeChunk];
   __shared__ float om[kMaxProbeChunk];
-  const int N = a.N, blocks = N * N / kTileThreads, block = blockIdx.x - ntiles;
+  const int N = a.N, blocks = N * N / kProbePixels, block = blockIdx.x - ntiles;
   const int chunk = block / blocks;
   const size_t plane = (size_t)N * N;
   const int s0 = chunk * a.chunk, s1 = min(a.nslot, s0 + a.chunk);
@@ -379,7 +381,7 @@ static __global__ void __launch_bounds__(kTileThreads, tile_min_blocks<kGatherRp
     om[i] = a.omax[s0 + i];
   }
   __syncthreads();
-  const int pix = (block % blocks) * kTileThreads + threadIdx.x;
+  const int pix = (block % blocks) * kProbePixels + threadIdx.x;
   const float2 q = a.quad[pix];
   const float2* obj = a.object + (size_t)(pix / N) * a.nxo + pix % N;
   KahanC acc[K];
@@ -446,7 +448,7 @@ static __global__ void __launch_bounds__(256) rpie_apply_kernel(RpieApplyArgs a)
 
 // One launch over `nchunk` chunks (K ≤ 4; N² is a multiple of 512 at every side).
 static inline void launch_probe_partial(const ProbeArgs& a, int nchunk, cudaStream_t s) {
-  const dim3 grid((a.N * a.N + 511) / 512, nchunk);
+  const dim3 grid(a.N * a.N / kProbePixels, nchunk);
   switch (a.K) {
     case 1: probe_partial_kernel<1><<<grid, 256, 0, s>>>(a); break;
     case 2: probe_partial_kernel<2><<<grid, 256, 0, s>>>(a); break;
@@ -565,8 +567,9 @@ static __global__ void __launch_bounds__(256) probe_norm_kernel(const float* par
   }
 }
 
-// Σ over chunks in order; mode 1: out = coef·Σ; 2: out += Σ compensated; 3: the blend P = (Σ + reg·P) / max(norm + reg, 1e-12) with reg = coef·max norm
-// (engine/ops.rs:371-381), `norm` one plane shared by the modes.
+// Σ over chunks in order; mode 1: out = coef·Σ; 2: out += Σ compensated; 3: the blend P = (Σ +
+// reg·P) / max(norm + reg, 1e-12) with reg = coef·max norm (engine/ops.rs:371-381), `norm` one
+// plane shared by the modes.
 static __global__ void probe_finalize_kernel(const float2* partial, int nchunk, int count,
                                       float2* probe, float2* out, float2* comp, float coef,
                                       int mode, const float* norm = nullptr,

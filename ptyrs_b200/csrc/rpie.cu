@@ -61,7 +61,8 @@ void rpie_batch(ptyb_handle* h, const ptyb_rpie_params& p, const int* frames, in
   const bool sum_probe = p.update_probe && !moved;
   int nchunk = 0;
   const int chunk = sum_probe ? probe_chunk(h, nslot, &nchunk) : 0;
-  const int tiles = p.update_object ? ntiles(h) : 0, pblocks = nchunk * (h->N * h->N / kTileThreads);
+  const int tiles = p.update_object ? ntiles(h) : 0;
+  const int pblocks = nchunk * (h->N * h->N / kProbePixels);
   if (tiles + pblocks > 0) {
     g.out = sums.num;
     g.pre = sums.den;
