@@ -2,7 +2,7 @@
 of slices, itself pinned to the reference's golden multislice runs): the LLK through the slices,
 LSQML epochs with every slice's step sizes, every slice and the probe, with and without the
 position model, on the far field of three slices with two unequal angular-spectrum gaps. Frame sides 64, 128 and 256 run the
-cluster sizes 1, 2 and 16."""
+default cluster sizes 1, 4 and 16 (the others built are in test_gpu_instances.py)."""
 import numpy as np
 import pytest
 

@@ -2,7 +2,8 @@
 as the reference holds its GPU engine to its CPU oracle (ptyrs/tests/engine_gpu.rs:160-165,
 298-322: relative error < 1e-4 on the LLK records and the final object and probe). One epoch
 of one batch is held to 1e-5 (FP32 against FP64 for one update); several epochs to 1e-4.
-Frame sides 64, 128 and 256 run the cluster sizes 1, 2 and 8."""
+Frame sides 64, 128 and 256 run the default cluster sizes 1, 4 and 16 (the others built are in
+test_gpu_instances.py)."""
 import numpy as np
 import pytest
 
