@@ -25,7 +25,8 @@ PTYB_D float2 cmulc_rn(float2 a, float2 b) {
   return make_float2(fmaf(a.x, b.x, a.y * b.y), fmaf(a.x, b.y, -(a.y * b.x)));
 }
 PTYB_HD float2 cscale(float2 a, float s) { return make_float2(a.x * s, a.y * s); }
-// conj(a) * b with the other product of the imaginary part fused: the probe sums' form.
+// conj(a) * b with the other product of the imaginary part fused: the probe sums' form, as accurate
+// as the one above, and kept apart from it for the same case's bits (fft.cuh, rotate_by).
 PTYB_D float2 cmulc_rn2(float2 a, float2 b) {
   return make_float2(fmaf(a.x, b.x, a.y * b.y), fmaf(-a.y, b.x, a.x * b.y));
 }

@@ -77,7 +77,7 @@ struct ptyb_handle {
   // Scratch, sized for `slots` frames per launch.
   int slots = 0;
   float2* upd = nullptr;      // [slots][K][N][N]
-  float2* field = nullptr;    // [slots][K][N][N]
+  float2* field = nullptr;    // [slots][max(K, 2)][N][N]
   float* icalc = nullptr;     // [slots][N][N]
   float* omax = nullptr;      // [slots]
   double* llk = nullptr;      // [P][4]

@@ -11,12 +11,13 @@
 // probes, the counts and the output touches global memory.
 //
 // What bounds it: latency. The exit waves' loads, the exchanges and the cluster barriers around
-// the transposes leave 37 % of the issue slots busy at 16 warps per SM (256² x 2), the memory
-// system under 25 %. Against the form it replaces (planes in shared memory for every step: 13
-// reads and 12 writes of each element per pass instead of 6.5 and 6.5, four global loads in
-// flight instead of 16) the passes take, per frame on one B200: gradient 256² x 2 3.53 -> 2.0 us,
-// carry 4.17 -> 2.27, LSQML 128² x 3 forward 0.77 -> 0.49 and backward 1.06 -> 0.63, amplitude
-// 96² x 2 0.83 -> 0.49, gradient 192² 1.53 -> 0.64, rPIE 64² 36 -> 13.5 us per batch of 100.
+// the transposes leave 34 % of the issue slots busy in the 256² x 2 gradient (24 warps per SM
+// allowed, 20 resident on average) and 35 % in the carry pass (16 and 14); DRAM moves 1.8 and 1.0
+// TB/s. Against the form it replaces (planes in shared memory for every step: 13 reads and 12
+// writes of each element per pass instead of 6.5 and 6.5, four global loads in flight instead of
+// 16) the passes take, per frame on one B200: gradient 256² x 2 3.53 -> 1.86 us, carry 4.17 ->
+// 2.19, LSQML 128² x 3 forward 0.77 -> 0.48 and backward 1.06 -> 0.62, amplitude 96² x 2 0.83 ->
+// 0.48, gradient 192² 1.53 -> 0.61, rPIE 64² 36 -> 12.8 us per batch of 100.
 //
 // Reference operators followed (physwkim/ptyrs): exit wave `obj_probe_to_psi`
 // (engine/ops.rs:47-71), unitary FFT (engine/fft.rs:155-234), the rPIE modulus
@@ -61,7 +62,8 @@ struct FrameArgs {
   const int* frames;     // frame of each slot of the launch
   const int2* corners;   // [nframe] window corner (x = oy, y = ox)
   float2* out;           // [slot][K][N][N] natural layout
-  float2* field;         // [slot][C][K·H][N] detector field in the CTA's strip layout
+  float2* field;         // [slot][C][K][E][T] detector field, thread by thread: written by the
+                         // pass before and read back by the same threads
   float* icalc;          // [slot][N][N] Σ_modes |Ψ|², detector layout
   float* omax;           // [slot] max |O|² over the window (object mode 0)
   double* llk;           // [slot][4] Poisson, Gaussian, Euclidian, photons

@@ -3,11 +3,11 @@
 // Object: one CTA owns half of a 16×16 square of the object and lists the launch's views that
 // overlap the square in ascending slot order (the reference's view order); four thread groups
 // per pixel take every fourth view of that list, each with Kahan-compensated float sums, and the
-// groups' sums are added in group order. No atomics touch the object and the result does not depend on
-// scheduling (the reference's tile-owned gather, ptyrs-kernels/src/lib.rs:388-437; operator
-// engine/ops.rs:282-310). Probe: the slots are cut
-// into chunks, each CTA sums one chunk in slot order for 512 probe pixels, and a second pass
-// adds the chunk sums in chunk order (engine/ops.rs:315-345).
+// groups' sums are added in group order. No atomics touch the object and the result does not
+// depend on scheduling (the reference's tile-owned gather, ptyrs-kernels/src/lib.rs:388-437;
+// operator engine/ops.rs:282-310). Probe: the slots are cut into chunks, each CTA sums one chunk
+// in slot order for 512 probe pixels, and a second pass adds the chunk sums in chunk order
+// (engine/ops.rs:315-345).
 #pragma once
 #include "common.cuh"
 
@@ -234,12 +234,16 @@ PTYB_D void object_tile(const GatherArgs& a) {
   }
 }
 
-// CTAs of 512 threads per SM a tile kernel is compiled for, by what a thread holds: 42 registers
-// for two views of up to two modes (ML 256² x 2 0.538 -> 0.460 us per frame, blend 0.477 -> 0.376,
-// 128² x 1 0.106 -> 0.071, against CTAs of 1024 with the mode count at run time; 64 registers
-// took 0.511, 0.375 and 0.077), 64 for rPIE's sums per mode of two modes and more (128² x 2 0.39
-// -> 0.29; at one mode 42 are ahead, 0.127 to 0.146), 32 for one view of three or four modes
-// (LSQML 128² x 3 0.265; 0.322 at 42 with two views).
+// CTAs of 512 threads per SM a tile kernel is compiled for, by what a thread holds, in us per frame
+// on one B200:
+// - three (40 registers) for two views of up to two modes: ML 256² x 2 0.462, blend 0.378, LSQML
+//   96² x 2 0.290, blend 128² x 1 0.072, with 16 to 44 bytes of spills at two modes; two CTAs (48
+//   to 60 registers, none spilled) take 0.512, 0.371, 0.350 and 0.087. CTAs of 1024 with the mode
+//   count at run time took 0.538 (ML), 0.477 and 0.106 (blends);
+// - two (up to 64) for rPIE's sums of two modes and more: 128² x 2 0.289, three CTAs 0.402 with 144
+//   bytes of spills; at one mode three are ahead, 64² 0.127 to 0.138;
+// - four (32) for one view of three or four modes: LSQML 128² x 3 0.218 with 24 bytes of spills,
+//   three CTAs with two views 0.322 with 94.
 template <int MODE, int K>
 __host__ __device__ constexpr int tile_min_blocks() {
   return MODE == kGatherRpie ? (K == 1 ? 3 : 2) : K <= 2 || MODE == kGatherBlend ? 3 : 4;

@@ -13,9 +13,9 @@ namespace ptyb {
 // num = −Σ 2·r·d, den = Σ 2·s·d + I·(2r/calc)². The b-term of den is linear in b, so it is
 // taken in the exit plane against the gradient pass's field (no transform of b). Shared memory
 // holds the K planes of a; the accumulators are each thread's pixels, in registers. Bound by the
-// latency of its loads (six arrays in the rows: 5.1 of 11.7 stalled warps per issue): 3.4 -> 2.6
-// us per frame of 256² x 2, 1.47 -> 1.11 at 192², against one plane at a time with the
-// accumulators in shared memory.
+// latency of its loads (six arrays in the rows: 4.0 of 10.4 stalled warps per issue) at 14 warps
+// per SM: 3.4 -> 2.39 us per frame of 256² x 2, 1.47 -> 0.935 at 192², against one plane at a time
+// with the accumulators in shared memory.
 struct GammaArgs {
   const float2* object;
   const float2* d_obj;

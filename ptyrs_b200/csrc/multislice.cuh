@@ -9,7 +9,7 @@
 // Backward: the field, the second xi pass, the residual, the inverse FFT and χ of the last
 // slice, then per gap back through conj(q·O) and the conjugate transfer function. The lines stay
 // in registers between the transposes (plane.cuh); per frame of 128² x 2 through three slices on
-// one B200: forward 1.96 -> 1.04 us, backward 2.65 -> 1.21 us.
+// one B200: forward 1.96 -> 1.01 us, backward 2.65 -> 1.14 us.
 #pragma once
 #include "frame.cuh"
 

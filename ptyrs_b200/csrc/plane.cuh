@@ -37,8 +37,10 @@ struct PlaneShape {
 // thread holds 16 elements, 1024 at side 64 (8 elements), two CTAs of 192 at 24 elements. A
 // kernel that holds little beside its line (`light`) takes 768 threads of 80 registers at side
 // 256: moves 0.906 -> 0.797 us per frame of 256² x 2, their spectra 0.998 -> 0.896, projection
-// 1.211 -> 1.055, gradient 1.941 -> 1.871, where the line search (2.46 -> 3.25), the carry pass
-// (2.21 -> 2.69) and at side 128 the LSQML passes (0.618 -> 0.757) spill and lose.
+// 1.211 -> 1.055, gradient 1.941 -> 1.871. Some spill a little there and gain all the same (bytes
+// stored: gradient 76, own moves and moves back 60, spectra 40 and 56, projection 4, the other
+// moves none). What holds more loses: line search 2.46 -> 3.25, carry pass 2.21 -> 2.69, at side
+// 128 the LSQML passes 0.618 -> 0.757; at 128 registers they spill 20, 104 and 0 bytes.
 template <int N, int C>
 __host__ __device__ constexpr int plane_min_blocks(bool light = false) {
   return N == 64 ? 2
