@@ -282,12 +282,12 @@ def sample_scan(s, m):
 # launch's frames.
 NCU_DRAM_BYTES_PER_FRAME = {
     # the 1000-frame cut of the ml256 scan, one 488-frame launch of each
-    "ml256": {"frame_ml_grad": 3.35e6, "deriv_sums": 1.06e6},
+    "ml256": {"frame_ml_grad": 3.41e6, "ml_gamma": 4.60e6, "deriv_sums": 1.07e6},
     # the carry pass on the 1024-frame cut of the dm256 scan
-    "dm256": {"frame_carry": 2.33e6},
+    "dm256": {"frame_carry": 2.28e6},
 }
-NCU_PROFILE = {"ml256": "profiles/ml_gradient_and_position_sums_ml256.md (a 1000-frame cut)",
-               "dm256": "profiles/dm256_launch_list.md (a 1024-frame cut)"}
+NCU_PROFILE = {"ml256": "profiles/plane_transforms_ml256.md (a 1000-frame cut)",
+               "dm256": "profiles/plane_transforms_ml256.md (a 1024-frame cut)"}
 
 
 def oracle_optics(s):
